@@ -525,9 +525,10 @@ int orac_gpu_server_stats(orac_gpu_server* s, int64_t* out8);
  * reference) ---------------------------------------------------------------
  * Lanes per i group on the M shell and on the L/H shells (16 or 32; 16 only
  * for groups of at most 4 atoms) and resident blocks per SM of its
- * forces-only build (5, 6 or 8); 0 selects the default of the context's mode
- * (alone 32, 32, 6; batched or served 16, 32, 8).  Forces, energies and
- * trajectories do not depend on it: only speed does. */
+ * forces-only build (5, 6 or 8); 0 selects the default (5 blocks; half warps
+ * on the M shell of contexts beside others and of large systems, whole warps
+ * otherwise).  Forces, energies and trajectories do not depend on it: only
+ * speed does. */
 int orac_gpu_set_pair_tuning(orac_gpu_ctx* ctx, int lpg_m, int lpg_lh,
                              int minb);
 /* The configuration in effect (lpg_m, lpg_lh, minb). */

@@ -102,6 +102,27 @@ int check_ready(orac_gpu_ctx* ctx) {
 
 }  // namespace
 
+// Launch configuration of the real-space kernel: the tuned one, or the
+// default.  The innermost shell's rows hold about a dozen groups: half a warp
+// each keeps the lanes busy, which is the faster form wherever there are rows
+// enough to fill the SMs (81,000 atoms: 1.02 against 1.16 ms a step).  A
+// context alone whose rows fit one wave of whole warps takes those, one pass
+// for every row (2,000 atoms: 234 against 254 us a step); a few blocks more
+// than a wave cost a launch half as much again.  5 blocks of 4 warps per SM
+// give the straight path the 96 registers it needs; 6 (80 registers) spills
+// and is slower with the device full (12 alchemical windows: 20.9 against
+// 19.9 ms for 12 steps), but takes the rows of 6 blocks per SM in one wave
+// (9,000 atoms, 750 blocks: 227 against 243 us a step).
+void pair_config(const orac_gpu_ctx* ctx, int* lpg, int* minb, bool m_shell) {
+  const int blocks = (ctx->G + 3) / 4;
+  const bool wave5 = blocks <= 5 * 148, wave6 = blocks <= 6 * 148;
+  if (m_shell)
+    *lpg = ctx->tune_lpg_m ? ctx->tune_lpg_m : (!ctx->shared_device && wave6 ? 32 : 16);
+  else
+    *lpg = ctx->tune_lpg_lh ? ctx->tune_lpg_lh : 32;
+  *minb = ctx->tune_minb ? ctx->tune_minb : (!ctx->shared_device && wave6 && !wave5 ? 6 : 5);
+}
+
 // Shell evaluation on device-resident coordinates (used by both ABIs).
 int shell_run(orac_gpu_ctx* ctx, char rshell, const double* d_xyz, const double* d_grp, const double* d_mol,
               double* d_f, double* d_e, double* d_stress, int energy) {
@@ -136,7 +157,7 @@ int shell_run_r(orac_gpu_ctx* ctx, char rshell, const ShellRadii& radii, const d
   PairArgs a;
   memset(&a, 0, sizeof(a));
   a.gpos = ctx->d_gpos;
-  a.gmeta = ctx->d_gmeta;
+  a.gmeta = ctx->d_gpair;
   a.aoff = ctx->d_aoff;
   a.atype = ctx->d_atype;
   a.apm = ctx->d_apm;
@@ -188,25 +209,17 @@ int shell_run_r(orac_gpu_ctx* ctx, char rshell, const ShellRadii& radii, const d
   a.natom = ctx->N;
   a.wcnt = ctx->d_wcnt;
   variant_fill(ctx, &a);
-  // launch configuration: the tuned one, or the mode's default -- the
-  // innermost shell's rows hold about a dozen groups: beside other contexts
-  // half a warp each (fewer instructions per row) and 8 blocks per SM, alone
-  // a warp each (twice the warps to hide one launch's latency) and 6
-  if (rshell == 'm')
-    a.lpg = ctx->tune_lpg_m ? ctx->tune_lpg_m : (ctx->shared_device ? 16 : 32);
-  else
-    a.lpg = ctx->tune_lpg_lh ? ctx->tune_lpg_lh : 32;
-  a.minb = ctx->tune_minb ? ctx->tune_minb : (ctx->shared_device ? 8 : 6);
-  // a row's entries split between two warps: only where twice the warps
-  // still fit in one wave (a launch of the M shell, which writes no next
-  // list, on a system of at most 1,024 groups); beyond that the second
-  // wave costs more than the shorter chains save
-  a.split = (rshell == 'm' && a.lpg == 32 && !a.next_on && !ctx->shared_device && ctx->G <= 1024) ? 2 : 1;
+  pair_config(ctx, &a.lpg, &a.minb, rshell == 'm');
+  a.early = (flags & SH_RELEASE) ? orac_early(ctx) : 0;
+  a.list_old = (flags & SH_LIST_OLD) ? 1 : 0;
   const bool want_e = (flags & SH_ENERGY) && d_e, want_s = (flags & SH_STRESS) && d_stress;
   a.energy = want_e ? 1 : 0;
   a.stress = want_s ? 1 : 0;
   // the forces-only build sums force_alchemy's dwrk where a schedule asks
   a.dwrk = (a.variant == VAR_ALCH && !want_e && !want_s) ? ctx->pair_dwrk : nullptr;
+  // its longest chains are the alchemical rows, which whole warps shorten
+  // (14,900 atoms: 1.90 against 2.02 ms a 15-fs step)
+  if (a.dwrk && !ctx->tune_lpg_m) a.lpg = 32;
   if (flags & SH_FIXED_OUT) a.ffix = reinterpret_cast<unsigned long long*>(d_f);
   if (want_e || want_s) CK(cudaMemsetAsync(ctx->d_acc, 0, ACC_N * sizeof(double), ctx->stream));
   if (!(flags & SH_PREPPED))
@@ -246,8 +259,8 @@ int orac_gpu_create(int device, orac_gpu_ctx** out) {
     return ORAC_ERR_CUDA;
   }
   if (dev_alloc(ctx, &ctx->d_acc, ACC_N) || dev_alloc(ctx, &ctx->d_red, 64) || dev_alloc(ctx, &ctx->d_total, 4) ||
-      dev_alloc(ctx, &ctx->d_flag, 4) || dev_alloc(ctx, &ctx->d_wcnt, 4) ||
-      cudaMemset(ctx->d_wcnt, 0, 4 * sizeof(unsigned long long)) != cudaSuccess) {
+      dev_alloc(ctx, &ctx->d_flag, 4) || dev_alloc(ctx, &ctx->d_wcnt, 4 * WCNT_SLOTS) ||
+      cudaMemset(ctx->d_wcnt, 0, 4 * WCNT_SLOTS * sizeof(unsigned long long)) != cudaSuccess) {
     orac_gpu_destroy(ctx);
     return ORAC_ERR_CUDA;
   }
@@ -260,7 +273,7 @@ int orac_gpu_destroy(orac_gpu_ctx* ctx) {
   cudaSetDevice(ctx->device);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   md_destroy(ctx);
-  void* ptrs[] = {ctx->d_gmeta, ctx->d_atype, ctx->d_apm, ctx->d_aq, ctx->d_aqd, ctx->d_amol, ctx->d_agrp,
+  void* ptrs[] = {ctx->d_gmeta, ctx->d_gpair, ctx->d_atype, ctx->d_apm, ctx->d_aq, ctx->d_aqd, ctx->d_amol, ctx->d_agrp,
                   ctx->d_gmol, ctx->d_amassinf, ctx->d_lj, ctx->d_ljd, ctx->d_exoff, ctx->d_exj, ctx->d_xyz, ctx->d_grp,
                   ctx->d_mol, ctx->d_gpos, ctx->d_aoff, ctx->d_ffix, ctx->d_acc, ctx->d_fout, ctx->d_red,
                   ctx->d_scan_tmp, ctx->d_total, ctx->d_flag, ctx->d_cell_of, ctx->d_cell_cnt, ctx->d_cell_start,
@@ -356,19 +369,14 @@ int orac_gpu_set_topology(orac_gpu_ctx* ctx, int ntap, int ngrp, int nprot, cons
     }
   // atoms whose type has no LJ partner at all: under lskip_ewald every pair
   // of theirs is skipped (src/force.f:416-417), and the pair kernel skips
-  // them without a table lookup; bit a of gmeta.y >> 16 marks atom a of the
-  // group as having LJ
+  // them without a table lookup
   {
     std::vector<unsigned char> tlj(ntype, 0);
     for (int t1 = 0; t1 < ntype; t1++)
       for (int t2 = 0; t2 < ntype; t2++)
         if (lj[t1 * (size_t)ntype + t2].y != 0.f) tlj[t1] = 1;
-    for (int g = 0; g < G; g++) {
-      int m = 0;
-      for (int a = 0; a < (gmeta[g].y & 0xff); a++)
-        if (tlj[nbtype[gmeta[g].x + a] - 1]) m |= 1 << a;
-      gmeta[g].y |= m << 16;
-    }
+    ctx->h_lj.resize(N);
+    for (int a = 0; a < N; a++) ctx->h_lj[a] = tlj[nbtype[a] - 1];
   }
   // exclusions: serial mapnl -> CSR with 0-based partners
   std::vector<int> exoff(N + 1), exj;
@@ -449,7 +457,7 @@ int orac_gpu_set_topology(orac_gpu_ctx* ctx, int ntap, int ngrp, int nprot, cons
   ctx->lists[1].off = ctx->lists[0].off;
   ctx->lists[2].off = ctx->lists[0].off;
   ctx->have_topo = true;
-  return ORAC_OK;
+  return pair_meta_build(ctx);
 }
 
 int orac_gpu_set_ewald(orac_gpu_ctx* ctx, int clewld, double alphal, int order, int nfft1, int nfft2, int nfft3,
@@ -576,10 +584,13 @@ void* orac_gpu_get_stream(orac_gpu_ctx* ctx) { return ctx ? (void*)ctx->stream :
 
 int orac_gpu_counters(orac_gpu_ctx* ctx, int64_t* out4, int reset) {
   if (!ctx) return ORAC_ERR_PARAM;
-  unsigned long long h[4];
+  unsigned long long h[4 * WCNT_SLOTS];
   CK(cudaStreamSynchronize(ctx->stream));
   CK(cudaMemcpy(h, ctx->d_wcnt, sizeof(h), cudaMemcpyDeviceToHost));
-  for (int k = 0; k < 4; k++) out4[k] = (int64_t)h[k];
+  for (int k = 0; k < 4; k++) {
+    out4[k] = 0;
+    for (int s = 0; s < WCNT_SLOTS; s++) out4[k] += (int64_t)h[4 * s + k];
+  }
   if (reset) CK(cudaMemset(ctx->d_wcnt, 0, sizeof(h)));
   return ORAC_OK;
 }

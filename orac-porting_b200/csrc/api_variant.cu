@@ -145,6 +145,29 @@ int alch_upload_tables(orac_gpu_ctx* ctx) {
 }
 
 
+int pair_meta_build(orac_gpu_ctx* ctx) {
+  const bool alch = ctx->variant == VAR_ALCH, rem = ctx->variant == VAR_REM;
+  std::vector<int4> gm(ctx->G);
+  for (int g = 0; g < ctx->G; g++) {
+    const int first = ctx->h_gfirst[g], n = ctx->h_gn[g];
+    int y = n | ctx->h_ss[first] << 4;
+    unsigned ty[2] = {0, 0};
+    for (int k = 0; k < n; k++) {
+      const int a = first + k;
+      if (alch ? ctx->h_softlj[a] : ctx->h_lj[a]) y |= 1 << (8 + k);
+      if (k < 4) {
+        ty[k / 2] |= (unsigned)(ctx->h_nbtype[a] - 1) << (16 * (k % 2));
+        if (rem && (ctx->h_vflag[a] & VF_REM)) y |= 1 << (GM_REM + k);
+      }
+      if (alch && ((ctx->h_vflag[a] & VF_MINF) || ctx->h_ssal[a] != 1)) y |= GM_SPECIAL;
+    }
+    gm[g] = make_int4(first, y, (int)ty[0], (int)ty[1]);
+  }
+  if (!ctx->d_gpair && dev_alloc(ctx, &ctx->d_gpair, gm.size())) return ORAC_ERR_CUDA;
+  CK(cudaMemcpy(ctx->d_gpair, gm.data(), gm.size() * sizeof(int4), cudaMemcpyHostToDevice));
+  return ORAC_OK;
+}
+
 void variant_fill(const orac_gpu_ctx* ctx, PairArgs* a) {
   a->variant = ctx->variant;
   if (ctx->variant == VAR_STD) return;
@@ -225,7 +248,7 @@ int orac_gpu_set_rem(orac_gpu_ctx* ctx, const int* rematom, int kind, double rem
     bump.arm();
     if (ctx->variant == VAR_REM) ctx->variant = VAR_STD;
     ctx->h_rem.clear();
-    return ORAC_OK;
+    return pair_meta_build(ctx);
   }
   if (kind < 0 || kind > 2) return ctx_fail(ctx, ORAC_ERR_PARAM, "REM segment kind %d (0, 1 or 2)", kind);
   if (!(rem_factor >= 0.0)) return ctx_fail(ctx, ORAC_ERR_PARAM, "rem_factor %g", rem_factor);
@@ -241,7 +264,7 @@ int orac_gpu_set_rem(orac_gpu_ctx* ctx, const int* rematom, int kind, double rem
   }
   if (int rc = build_vflag(ctx)) return rc;
   ctx->variant = VAR_REM;
-  return ORAC_OK;
+  return pair_meta_build(ctx);
 }
 
 int orac_gpu_set_rem_factor_async(orac_gpu_ctx* ctx, double rem_factor, void* stream) {
@@ -265,7 +288,7 @@ int orac_gpu_set_alchemy(orac_gpu_ctx* ctx, const int* ss_alchemy, const double*
     bump.arm();
     if (ctx->variant == VAR_ALCH) ctx->variant = VAR_STD;
     ctx->h_ssal.clear();
-    return ORAC_OK;
+    return pair_meta_build(ctx);
   }
   if (!rmin || !epsm) return ctx_fail(ctx, ORAC_ERR_PARAM, "rmin and epsm are required");
   const int N = ctx->N;
@@ -289,8 +312,11 @@ int orac_gpu_set_alchemy(orac_gpu_ctx* ctx, const int* ss_alchemy, const double*
   ctx->at.qsoft = qsoft;
   ctx->at.ljsoft = ljsoft;
   ctx->at.opls = opls ? 1 : 0;
+  ctx->h_softlj.resize(N);
+  for (int a = 0; a < N; a++) ctx->h_softlj[a] = sf[a].y != 0.f;
   if (int rc = build_vflag(ctx)) return rc;
   ctx->variant = VAR_ALCH;
+  if (int rc = pair_meta_build(ctx)) return rc;
   const double zero[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   return orac_gpu_set_lambda(ctx, zero, 0, 0, nullptr);
 }

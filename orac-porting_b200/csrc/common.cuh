@@ -38,6 +38,9 @@ enum {
   ACC_N = 27
 };
 
+// copies of the pair kernel's work counters
+constexpr int WCNT_SLOTS = 64;
+
 // Kernel families that the launch profiler brackets with CUDA events: the
 // real-space pair kernel, the drift and kick kernels of the integrator, one
 // SPME evaluation (spread to gather, as one interval), the bonded kernel.
@@ -95,11 +98,17 @@ struct ShellRadii {
   double rcutm, rtolm, rneim, rcutl, rtoll, rneil, rcuth, rtolh, rneih;
 };
 
+// The pair kernel's record of a group (d_gpair): x first atom, y natoms (4
+// bits) | ss type << 4 | 8 bits of atoms with LJ << 8 | for groups of up to 4
+// atoms their REM flags << GM_REM | GM_SPECIAL with an alchemical or
+// fixed-mass atom; z, w the LJ types of up to 4 atoms, 16 bits each.
+constexpr int GM_REM = 16, GM_SPECIAL = 1 << 20;
+
 // Arguments of one pair-kernel launch (passed by value).
 struct PairArgs {
   // topology
   const double4* gpos;   // [G] scaled group centres (.w unused)
-  const int2* gmeta;     // [G] (first atom, natoms | ss_type << 8)
+  const int4* gmeta;     // [G] GM_* (ctx->d_gpair)
   const float4* aoff;    // [N] Cartesian offset from group centre, charge
   const int* atype;      // [N] 0-based LJ type
   const float* apm;      // [N] mass fraction in group
@@ -133,18 +142,21 @@ struct PairArgs {
   double* acc;               // [ACC_N]
   int natom;
   // work counters: list entries scanned, entries kept for the next shell,
-  // atom pairs evaluated with Ewald, atom pairs evaluated LJ-only
+  // atom pairs evaluated with Ewald, atom pairs evaluated LJ-only, in
+  // WCNT_SLOTS copies that orac_gpu_counters adds up
   unsigned long long* wcnt;
   // 0: skip the image term of the molecular virial and the block reduction
   // (MD without pressure coupling needs neither)
   int stress;
-  // lanes that own one i group: 32, or 16 (two groups per warp) for lists
-  // with short rows; 16 applies to groups of at most 4 atoms
+  // lanes that own one i group: 32, or 16 (two groups per warp); 16 applies
+  // to groups of at most 4 atoms
   int lpg;
   // resident blocks per SM of the forces-only build (5, 6 or 8)
   int minb;
-  // warps per row (1, or 2 for whole-warp rows without a next-shell list)
-  int split;
+  // the next grid released at the start (pdl_release); the list is older than
+  // the kernel before this launch, so that its first entries may be read
+  // before the wait
+  int early, list_old;
   // variant (VAR_*); REM: seg_select kind and rem_factor(3)
   int variant;
   const unsigned char* vflag;  // [N]
@@ -202,7 +214,9 @@ enum {
   SH_STRESS = 2,    // molecular virial (finalize + image term)
   SH_PREPPED = 4,   // gpos/aoff already written and the force accumulator zeroed
   SH_FIXED_OUT = 8, // d_f is a fixed-point accumulator: skip finalize
-  SH_NO_NEXT = 16   // write no next-shell list (a later pass rebuilds it)
+  SH_NO_NEXT = 16,  // write no next-shell list (a later pass rebuilds it)
+  SH_RELEASE = 32,  // release the kernel that follows early (pdl_release)
+  SH_LIST_OLD = 64  // the shell's list was written before the preceding kernel
 };
 
 struct PmePlan {
@@ -288,9 +302,8 @@ struct orac_gpu_ctx {
   unsigned param_gen = 0;
   // pair-kernel launch configuration (orac_gpu_set_pair_tuning, the
   // autotuner): lanes per i group on the M shell and on the L/H shells,
-  // resident blocks per SM; 0 = the default for the context's mode (alone:
-  // 32, 32, 6; beside other contexts: 16, 32, 8).  Results do not depend on
-  // it (fixed-point sums)
+  // resident blocks per SM; 0 = the default (pair_config).  Results do not
+  // depend on it (fixed-point sums)
   int tune_lpg_m = 0, tune_lpg_lh = 0, tune_minb = 0;
   std::unordered_map<void*, size_t> dmem;  // live device allocations
   size_t dmem_bytes = 0;
@@ -312,11 +325,14 @@ struct orac_gpu_ctx {
   std::vector<unsigned char> h_intra_b, h_intra_p;
   std::vector<double> h_charge, h_mass;
   std::vector<int> h_ss, h_nbtype;
+  std::vector<unsigned char> h_lj;      // atoms whose type has an LJ partner
+  std::vector<unsigned char> h_softlj;  // atoms with a soft-core epsilon (alchemy)
   std::vector<double> h_ecc12, h_ecc6;
   ApiScratch api;
 
   // device topology
   int2* d_gmeta = nullptr;
+  int4* d_gpair = nullptr;  // the pair kernel's record of each group (GM_*)
   int* d_atype = nullptr;
   float* d_apm = nullptr;
   float* d_aq = nullptr;
@@ -417,7 +433,7 @@ struct orac_gpu_ctx {
 
   // measurement: work counters of the pair kernel and CUDA events around
   // its launches (recorded into captured graphs as event nodes)
-  unsigned long long* d_wcnt = nullptr;  // [4]
+  unsigned long long* d_wcnt = nullptr;  // [4 WCNT_SLOTS]
   int prof = 0;           // mask of the profiled kernel families (PROF_*)
   bool prof_bad = false;  // an event pair could not be timed
   std::vector<cudaEvent_t> prof_ev;  // pairs (start, end)
@@ -440,6 +456,9 @@ struct ParamGenBump {
   }
 };
 
+// the kernels of a step may release their successors early (pdl_release)
+static inline int orac_early(const orac_gpu_ctx* ctx) { return ctx->shared_device ? 0 : 1; }
+
 // record the start/end events of one profiled launch of a family (no-op
 // unless that family is profiled)
 int prof_begin(orac_gpu_ctx* ctx, int* slot, int family = PROF_PAIR);
@@ -452,6 +471,8 @@ int prof_collect(orac_gpu_ctx* ctx, int a, int b);
 void variant_fill(const orac_gpu_ctx* ctx, PairArgs* a);
 int variant_out_launch(orac_gpu_ctx* ctx, int forces_on);
 void variant_free(orac_gpu_ctx* ctx);
+// rebuild d_gpair after the topology or the variant changed
+int pair_meta_build(orac_gpu_ctx* ctx);
 
 // ---------------------------------------------------------------- errors
 int ctx_fail(orac_gpu_ctx* c, int code, const char* fmt, ...);
@@ -519,10 +540,19 @@ static inline cudaError_t orac_launch(void (*kernel)(KArgs...), dim3 grid, dim3 
 }
 
 // Wait for the grids this one depends on (their memory operations complete
-// and visible).  The next grid is released when this one completes: blocks
-// released earlier would hold SM slots while they wait, which costs the
-// concurrent systems of a batch more than it saves.
+// and visible).
 __device__ __forceinline__ void pdl_enter() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Release the next grid of the stream: its blocks are scheduled once every
+// block of this one has got here, and what they do before their own pdl_enter
+// (launch, loads of data that no running kernel writes) overlaps this grid.
+// Only after pdl_enter, so that all grids before this one are complete by
+// then, and only in a context alone on its device (orac_early): released
+// blocks hold SM slots while they wait, which costs the concurrent systems of
+// a batch more than it saves.
+__device__ __forceinline__ void pdl_release(int early) {
+  if (early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 // ------------------------------------------------------ internal drivers
 // k_list.cu
@@ -605,6 +635,7 @@ int bonded_launch(orac_gpu_ctx* ctx, int mask, const double* d_x, double* d_f, u
 void bonded_free(orac_gpu_ctx* ctx);
 int bonded_set_constraints(orac_gpu_ctx* ctx, const int* cnst, int ncnst);
 // api.cu
+void pair_config(const orac_gpu_ctx* ctx, int* lpg, int* minb, bool m_shell);
 int shell_run(orac_gpu_ctx* ctx, char rshell, const double* d_xyz,
               const double* d_grp, const double* d_mol, double* d_f,
               double* d_e, double* d_stress, int energy);

@@ -14,22 +14,25 @@
 //      entry's mask, src/force.f:396-731;
 //   4. for switched pairs adds the S'(R) V_ij term distributed by mass
 //      fraction, src/force.f:754-817.
-// Steps 1-2 run a lane per list entry; step 3 a lane per j atom of the
-// in-band entries, queued in shared memory (k_pair below).  Forces go to
+// Steps 1-2 run a lane per list entry; steps 3-4 a lane per in-band entry,
+// queued in shared memory (k_pair below).  Forces go to
 // 64-bit fixed-point accumulators with atomics, so the sum is independent
 // of the order of the atomics.
 // The molecular virial is assembled without per-pair work: ORAC's
 // sum_pairs f (x) (Rm_i - Rm_j - img) equals sum_atoms F_a (x) Rm_a (done in
 // the finalize kernel) plus, for pairs that cross the box, G_ij (x) co.img
 // where G_ij is the pair's total force on the j group (done here).
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace {
 
-constexpr int WPB = 4;  // warps per block
+// warps per block: 4; 2 for groups of more than 4 atoms, whose lanes keep
+// more in shared memory
+__host__ __device__ constexpr int warps_per_block(int mg) { return mg > 4 ? 2 : 4; }
 constexpr float AS_A1 = 0.2548296f, AS_A2 = -0.28449674f, AS_A3 = 1.4214137f;
 constexpr float AS_A4 = -1.453152f, AS_A5 = 1.0614054f, AS_QP = 0.3275911f;
-constexpr int LJ_SMEM_MAX = 2048;  // staged LJ table entries: 16 KB beside the static queues
 
 __device__ __forceinline__ long long to_fix(float v) { return __float2ll_rn(v * (float)ORAC_FSCALE); }
 
@@ -38,43 +41,19 @@ __device__ __forceinline__ void fix_add(unsigned long long* p, float v) {
   if (q != 0) atomicAdd(p, (unsigned long long)q);
 }
 
-// sum over the aligned runs of W lanes of a warp
-template <int W>
-__device__ __forceinline__ float seg_sum(float v) {
-#pragma unroll
-  for (int o = W / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
+// The force path's products and sums with their rounding spelled out: every
+// build of the kernel (with energies or without, any lanes per row) then gives
+// the same forces bit for bit, and an energy step or a restart does not change
+// a trajectory.
+__device__ __forceinline__ float fm(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ float mu(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float ad(float a, float b) { return __fadd_rn(a, b); }
 
-// Sum of P values over the aligned runs of W lanes, scattered: at each
-// shuffle step a lane keeps half of its values and receives the matching
-// half of its partner's, so P - 1 shuffles (plus log2(W / P) for the last
-// value) replace P full butterflies.  Returns the segment's total of value
-// rs_index<W, P>(lane % W).
-template <int W, int P, typename T>
-__device__ __forceinline__ T reduce_scatter(T (&v)[P], int sl) {
-#pragma unroll
-  for (int h = P / 2, o = W / 2; h >= 1; h >>= 1, o >>= 1) {
-    const bool up = (sl & o) != 0;
-#pragma unroll
-    for (int k = 0; k < h; k++) {
-      const T send = up ? v[k] : v[k + h];
-      const T keep = up ? v[k + h] : v[k];
-      v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-    }
-  }
-  T r = v[0];
-#pragma unroll
-  for (int o = W / P / 2; o >= 1; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
-  return r;
-}
-
-template <int W, int P>
-__device__ __forceinline__ int rs_index(int sl) {
-  int idx = 0;
-#pragma unroll
-  for (int o = W / 2, h = P / 2; h >= 1; o >>= 1, h >>= 1) idx += (sl & o) ? h : 0;
-  return idx;
+// 2^x by the hardware instruction
+__device__ __forceinline__ float ex2f(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
 }
 
 __device__ __forceinline__ double warp_sumd(double v) {
@@ -266,169 +245,160 @@ __device__ __forceinline__ void alch_energy_fp64(const PairArgs& A, double rx, d
 }
 
 
-// Ring capacities of the per-group queues (LPG lanes own one i group).
-// Entries: at most LPG - 1 left over from the previous chunk plus LPG new.
-// Atom slots: at most LPG - 1 left over plus LPG entries of MG atoms.
-template <int MG, int LPG>
-struct Rings {
-  static constexpr int QE = 2 * LPG;
-  static constexpr int need = LPG - 1 + LPG * MG;
-  static constexpr int QS = need <= 64 ? 64 : (need <= 128 ? 128 : (need <= 256 ? 256 : 512));
+// Entry queue of one i group: at most LPG - 1 entries left over from the
+// chunks before plus LPG new ones.
+template <int LPG>
+struct Queue {
+  static constexpr int N = 2 * LPG;
 };
 
-// A slot names one j atom of a queued entry: entry (6 bits), its position t
-// among the entry's slots (3), its atom b in the j group (3), the entry's
-// slot count - 1 (3).
-__device__ __forceinline__ unsigned short slot_pack(int e, int t, int b, int n) {
-  return (unsigned short)(e | (t << 6) | (b << 9) | ((n - 1) << 12));
-}
-
-// LPG lanes own one i group for a whole list row: 32 (a warp) for the long
-// rows of the L and H lists, 16 (two groups per warp) for the short rows of
-// the M list, where a full warp would leave most lanes idle.
+// LPG lanes own one i group for a whole list row (two groups per warp at 16).
 //
 // Phase 1 (a lane per list entry, LPG entries per chunk): FP64 minimum image
-// and band of the group pair, the next shell's list entry, and, for an
-// in-band entry, its geometry (FP32 centre distance, S, S', and in FP64 what
-// the energies need) into the group's entry queue and one slot per j atom to
-// evaluate into its slot queue (order kept by ballots and a segment scan).
+// and band of the group pair, the next shell's list entry (order kept by
+// ballots), and, for an in-band entry with a pair to evaluate, its geometry
+// (FP32 centre distance, S, S', and in FP64 what the energies need) and the
+// bits of its atom pairs into the row's queue in shared memory.
 //
-// Phase 2 (a lane per j atom): passes of up to LPG slots that hold whole
-// entries.  A lane takes its j atom's offset and charge once and runs over
-// the i atoms (broadcast reads of shared memory): the j atom's force sums in
-// the lane, and goes out with one fixed-point atomic per component, S'(R) V
-// term included; the entry's V is a segmented shuffle sum over the entry's
-// lanes.  The i atoms' forces sum per lane across passes and leave by one
-// segment reduction at the end of the row.
+// Phase 2 (a lane per queued entry, full passes of LPG entries and one for
+// the row's rest): the lane evaluates every atom pair of its two groups, the
+// i atoms from shared memory (a broadcast), the j atoms from memory once.
+// Forces of both groups and V sum in the lane in a fixed order, so neither
+// LPG nor the order of the passes changes a result; the S'(R) V term needs no
+// exchange between lanes.  The j atoms leave by one fixed-point atomic per
+// component and entry; the i atoms are added in fixed point over the row's
+// passes and leave by one reduction over the lanes at the end of the row.
+//
+// What bounds it: on one system latency (a row is one pass of the M shell,
+// two of the L shell), with the device full the issue of the pair arithmetic.
+// A lane per entry keeps the pair arithmetic free of queue bookkeeping: the
+// lane-per-j-atom form before it spent 4.4 M warp instructions on the M shell
+// of 3,000 waters, two thirds of them on slots, shuffles and reductions.
 //
 // MINB: resident blocks per SM the forces-only build is compiled for (5, 6
-// or 8; fewer registers per thread the more blocks); a context alone favours
-// one launch's latency, contexts sharing the device more warps per SM.
+// or 8; fewer registers per thread the more blocks).
 template <int MG, bool EN, int VAR, int LPG, int MINB>
-__global__ void __launch_bounds__(WPB * 32, MINB) k_pair(const PairArgs A) {
-  pdl_enter();
+__global__ void __launch_bounds__(warps_per_block(MG) * 32, MINB) k_pair(const PairArgs A) {
+  constexpr int WPB = warps_per_block(MG);
   // the alchemy variant, and its build that also sums force_alchemy's dwrk
   constexpr bool ALCH = VAR == VAR_ALCH || VAR == VAR_ALCHW;
   constexpr int SEG = 32 / LPG;  // groups per warp
-  constexpr int QE = Rings<MG, LPG>::QE, QS = Rings<MG, LPG>::QS;
+  constexpr int QE = Queue<LPG>::N;
   constexpr int NQ = WPB * SEG;  // groups per block
   constexpr unsigned FULL = 0xffffffffu;
-  extern __shared__ float2 s_lj[];
+  // pair bits: a * 8 + b, as the list's masks have them; four atoms a group
+  // fit the low word
+  using Bits = typename std::conditional<(MG > 4), unsigned long long, unsigned>::type;
+  constexpr Bits COLS = (Bits)0x0101010101010101ull;
   __shared__ float4 s_ai[NQ][MG];
   __shared__ int s_ti[NQ][MG];  // the i atom's row of the LJ tables (type * ntype)
   __shared__ float s_pm[NQ][MG];
   __shared__ double s_qd[NQ][EN ? MG : 1];
   __shared__ int s_fi[NQ][VAR != VAR_STD ? MG : 1];
   __shared__ float2 s_sf[NQ][ALCH ? MG : 1];
-  // entry queue: centre distance and S, S', j group metadata, skip mask;
-  // FP64 distance and S and the Cartesian image for the energy build
+  // entry queue: centre distance and S; first j atom, j group metadata, S';
+  // pair bits; FP64 distance and S and the Cartesian image for the energies
   __shared__ float4 s_edc[NQ][QE];
+  __shared__ int4 s_emeta[NQ][QE];
   __shared__ float s_edsw[NQ][QE];
-  __shared__ int2 s_emeta[NQ][QE];
-  __shared__ unsigned long long s_emsk[NQ][QE];
+  __shared__ Bits s_ebits[NQ][QE];
   __shared__ double4 s_ecd[EN ? NQ : 1][EN ? QE : 1];
-  __shared__ float4 s_eimg[EN ? NQ : 1][EN ? QE : 1];
-  __shared__ unsigned short s_slot[NQ][QS];
-  __shared__ double s_red[WPB][ACC_N];
-  __shared__ double s_vimg[WPB][9];
+  __shared__ double4 s_eimg[EN ? NQ : 1][EN ? QE : 1];
+  // the i atoms' forces of each lane's entries, in fixed point (a row of
+  // lanes per value; the padding puts the values a lane apart in the banks)
+  __shared__ long long s_fiq[3 * MG][WPB * 32 + 2];
+  __shared__ double s_red[EN ? WPB : 1][18];
+  __shared__ unsigned s_cnt[WPB][3];
   __shared__ float s_af[ALCH ? 2 : 1][9], s_afq[ALCH ? 2 : 1][9];
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int sub = lane / LPG, sl = lane % LPG, q = warp * SEG + sub;
   const unsigned below = (1u << sl) - 1u;  // lanes of this segment below this one
   const int seg0 = sub * LPG;              // first lane of this segment
-  const int nt2 = A.ntype * A.ntype;
-  const bool staged = nt2 <= LJ_SMEM_MAX;
-  if (threadIdx.x < WPB * 9) s_vimg[threadIdx.x / 9][threadIdx.x % 9] = 0.0;
-  if (staged)
-    for (int k = threadIdx.x; k < nt2; k += blockDim.x) s_lj[k] = A.lj[k];
+  const float2* __restrict__ lj = A.lj;
+  // the row and its first entries: with list_old they are older than the
+  // kernel before this one, and read before the wait for it
+  if (!A.list_old) pdl_enter();
+  const int i = (blockIdx.x * WPB + warp) * SEG + sub;
+  const bool gvalid = i < A.ngrp;
+  const int4 mi = gvalid ? A.gmeta[i] : make_int4(0, 0, 0, 0);
+  const int row = gvalid ? A.off[i] : 0, m = gvalid ? A.cnt[i] : 0;
+  int jnext = 0;  // the lane's entry of the chunk to come
+  unsigned long long mnext = 0ull;
+  if (sl < m) {
+    jnext = A.lj_[row + sl];
+    mnext = A.lmask[row + sl];
+  }
+  if (A.list_old) pdl_enter();
+  pdl_release(A.early);
   if constexpr (ALCH) {  // the current lambda tables
     if (threadIdx.x < 18) {
       s_af[threadIdx.x / 9][threadIdx.x % 9] = A.ad->af[threadIdx.x / 9][threadIdx.x % 9];
       s_afq[threadIdx.x / 9][threadIdx.x % 9] = A.ad->afq[threadIdx.x / 9][threadIdx.x % 9];
     }
+    __syncthreads();
   }
-  __syncthreads();
-  const float2* lj = staged ? s_lj : A.lj;
-  // under lskip_ewald an atom without LJ has no pair to evaluate
-  const bool ljonly = !ALCH && A.lskip && A.ewald;
+  // under lskip_ewald only pairs of atoms with LJ are evaluated
+  const bool ljonly = A.lskip && A.ewald;
   const float remf = VAR == VAR_REM ? __ldg(A.remf) : 1.f;  // rem_factor(3)
+  const float asqp = AS_QP * A.alphal;                      // A&S: t = 1 / (1 + p alpha r)
+  const float a2l2 = -A.alphal * A.alphal * 1.44269504f;    // exp(-(alpha r)^2) as a power of two
+  const float twa = A.twrtpi * A.alphal;
   // this segment's bits of a warp ballot
   auto segbits = [&](unsigned b) -> unsigned { return SEG == 1 ? b : (b >> seg0) & 0xffffu; };
 
   double ec0 = 0, ec1 = 0, ec2 = 0, eq0 = 0, eq1 = 0, eq2 = 0;
   double ex0 = 0, ex1 = 0, ex2 = 0;  // variant sums (ACC_X)
+  // image term of the molecular virial (stress only)
+  double vimg[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   // force_alchemy's dwrk of a forces-only launch under a schedule (A.dwrk):
   // U(lambda) - U(lambda0) of the alchemical pairs, FP64 on the FP32 pair
   // geometry (the other pairs' terms are equal at lambda and lambda0)
   double wk = 0.0;
   unsigned npairs = 0, nscan = 0, nkept = 0;
-  // image term of the molecular virial: each pass's per-lane FP32 terms are
-  // summed over the warp in FP64 into this warp's accumulator (stress only;
-  // the terms cancel heavily, so no FP32 sums across lanes)
-  float vimg[9];
-#pragma unroll
-  for (int c = 0; c < 9; c++) vimg[c] = 0.f;
-  auto flush_vimg = [&]() {  // every lane of the warp calls it
-#pragma unroll
-    for (int c = 0; c < 9; c++) {
-      const double t = warp_sumd((double)vimg[c]);
-      if (lane == 0) s_vimg[warp][c] += t;
-      vimg[c] = 0.f;
-    }
-  };
 
-  // every lane of a warp runs the same trip counts, so the warp-wide
-  // ballots and shuffles stay convergent
-  // a row split between two warps (A.split = 2, whole-warp rows of a
-  // launch that writes no next-shell list): each takes a chunk-aligned half
-  // of the entries, and both add the i atoms' forces by exact fixed-point
-  // atomics, so the row's result does not change; its chain is half as long
-  const int split = SEG == 1 ? A.split : 1;
-  for (int pw = blockIdx.x * WPB + warp; pw * SEG < A.ngrp * split; pw += gridDim.x * WPB) {
-    const int gw = split == 2 ? pw >> 1 : pw;
-    const int part = pw - gw * split;
-    const int i = gw * SEG + sub;
-    const bool gvalid = i < A.ngrp;
-    const int2 mi = gvalid ? A.gmeta[i] : make_int2(0, 0);
-    const int ifirst = mi.x, ni = mi.y & 0xff, typei = (mi.y >> 8) & 0xff, ljmi = mi.y >> 16;
+  // every lane of a warp runs the same trip counts, so the warp-wide ballots
+  // and shuffles stay convergent
+  {
+    const int ifirst = mi.x, ni = mi.y & 15, typei = (mi.y >> 4) & 15, ljmi = (mi.y >> 8) & 0xff;
     const double4 gi = gvalid ? A.gpos[i] : make_double4(0.0, 0.0, 0.0, 0.0);
-    const int row = gvalid ? A.off[i] : 0, mrow = gvalid ? A.cnt[i] : 0;
-    // this warp's entries [k0, m) of the row
-    const int chunk = split == 2 ? ((mrow + 1) / 2 + LPG - 1) / LPG * LPG : mrow;
-    const int k0 = min(mrow, part * chunk), m = min(mrow, k0 + chunk);
     int mmax = m;
     if (SEG == 2) mmax = max(mmax, __shfl_xor_sync(FULL, m, 16));
-    if (sl < ni) {
-      s_ai[q][sl] = A.aoff[ifirst + sl];
-      s_ti[q][sl] = A.atype[ifirst + sl] * A.ntype;
-      s_pm[q][sl] = A.apm[ifirst + sl];
-      if (EN) s_qd[q][sl] = A.qd[ifirst + sl];
-      if (VAR != VAR_STD) s_fi[q][sl] = A.vflag[ifirst + sl];
-      if (ALCH) s_sf[q][sl] = A.soft[ifirst + sl];
+    if (sl < MG) {  // (slots beyond the group's atoms: zeros, type 0)
+      const bool in = sl < ni;
+      const int at = ifirst + sl;
+      s_ai[q][sl] = in ? A.aoff[at] : make_float4(0.f, 0.f, 0.f, 0.f);
+      s_ti[q][sl] = in ? A.atype[at] * A.ntype : 0;
+      s_pm[q][sl] = in ? A.apm[at] : 0.f;
+      if (EN) s_qd[q][sl] = in ? A.qd[at] : 0.0;
+      if (VAR != VAR_STD) s_fi[q][sl] = in ? A.vflag[at] : 0;
+      if (ALCH) s_sf[q][sl] = in ? A.soft[at] : make_float2(0.f, 0.f);
     }
-    __syncwarp();
-    // the i atoms' forces of this lane's pairs and S'V shares, in fixed
-    // point: integer sums are exact, so the row's total does not depend on
-    // which lane took which j atom (half or full warps, any block shape)
-    long long fiq[MG][3];
+    Bits irows = 0;  // the i atoms to evaluate, a byte each
 #pragma unroll
-    for (int a = 0; a < MG; a++) fiq[a][0] = fiq[a][1] = fiq[a][2] = 0ll;
+    for (int a = 0; a < MG; a++)
+      if (a < ni && (!ljonly || ((ljmi >> a) & 1))) irows |= (Bits)0xff << (8 * a);
+    __syncwarp();
+    // the i atoms' forces are added over the lane's entries in fixed point,
+    // in shared memory: integer sums are exact, so the row's total does not
+    // depend on which lane took which entry
+    bool started = false;  // a pass of this row has run
 
     int nout = 0;
     int qh = 0, qn = 0;  // entry queue: head, entries pending
-    int sh = 0, sn = 0;  // slot queue: head, slots pending
-    for (int base = k0; base < mmax; base += LPG) {
+    for (int base = 0; base < mmax; base += LPG) {
       // ---- phase 1: geometry of list entry k (src/force.f:265-333)
       const int k = base + sl;
       const bool valid = k < m;
-      int j = 0;
-      unsigned long long msk = 0ull;
-      int2 mj = make_int2(0, 0);
+      const int j = jnext;
+      const unsigned long long msk = mnext;
+      if (k + LPG < m) {
+        jnext = A.lj_[row + k + LPG];
+        mnext = A.lmask[row + k + LPG];
+      }
+      int4 mj = make_int4(0, 0, 0, 0);
       double drj = 1e300, cx = 0.0, cy = 0.0, cz = 0.0, imx = 0.0, imy = 0.0, imz = 0.0;
       if (valid) {
-        j = A.lj_[row + k];
-        msk = A.lmask[row + k];
         const double4 gj = A.gpos[j];
         mj = A.gmeta[j];
         double dx = gi.x - gj.x, dy = gi.y - gj.y, dz = gi.z - gj.z;
@@ -438,10 +408,10 @@ __global__ void __launch_bounds__(WPB * 32, MINB) k_pair(const PairArgs A) {
         dx -= imx;
         dy -= imy;
         dz -= imz;
-        cx = A.c11 * dx + A.c12 * dy + A.c13 * dz;
-        cy = A.c22 * dy + A.c23 * dz;
-        cz = A.c33 * dz;
-        drj = cx * cx + cy * cy + cz * cz;
+        cx = __fma_rn(A.c13, dz, __fma_rn(A.c12, dy, __dmul_rn(A.c11, dx)));
+        cy = __fma_rn(A.c23, dz, __dmul_rn(A.c22, dy));
+        cz = __dmul_rn(A.c33, dz);
+        drj = __fma_rn(cz, cz, __fma_rn(cy, cy, __dmul_rn(cx, cx)));
       }
       if (A.next_on) {  // the next inner shell's list, order kept (src/force.f:279-286)
         const bool keep = valid && drj < A.r2neigh;
@@ -456,13 +426,16 @@ __global__ void __launch_bounds__(WPB * 32, MINB) k_pair(const PairArgs A) {
       nscan += valid ? 1u : 0u;
       if (!A.forces_on) continue;
       // band: non-switched [rinn0, rout), S on [rout, rout0), 1-S on [rinn, rinn0)
-      bool inb = false;
+      Bits bits = 0;
       float sw = 1.f, dsw = 0.f;
       double swd = 1.0;
       if (valid) {
         const bool sw_out = drj >= A.r2out && drj < A.r2out0;
         const bool sw_in = drj >= A.r2inn && drj < A.r2inn0;
-        inb = (drj >= A.r2inn0 && drj < A.r2out) || sw_out || sw_in;
+        if ((drj >= A.r2inn0 && drj < A.r2out) || sw_out || sw_in) {
+          const unsigned cols = ljonly ? (unsigned)(mj.y >> 8) & 0xffu : (1u << (mj.y & 15)) - 1u;
+          bits = ~(Bits)msk & irows & ((Bits)cols * COLS);
+        }
         if (sw_out || sw_in) {
           // S(R) of src/force.f:311-317 for the forces: FP32 arithmetic on
           // the two factors taken in FP64, the distance to the band edge
@@ -479,13 +452,13 @@ __global__ void __launch_bounds__(WPB * 32, MINB) k_pair(const PairArgs A) {
           const float iars2f = sw_out ? A.iarsout2 : A.iarsinn2;
           const float sgn = sw_out ? 1.f : -1.f;
           double y = (double)rsqrtf((float)drj);
-          y = y * (1.5 - 0.5 * drj * y * y);
-          const double rspd = drj * y;
-          const float auxa = (float)((ars1 + 2.0 * rspd) * iars2);
-          const float auxb = (float)(edge - rspd);
-          const float s3 = auxa * auxb * auxb;
-          sw = sw_out ? s3 : 1.0f - s3;
-          dsw = sgn * (-2.0f * auxa * auxb + 2.0f * auxb * auxb * iars2f) * (float)y;
+          y = __dmul_rn(y, __fma_rn(__dmul_rn(-0.5 * drj, y), y, 1.5));
+          const double rspd = __dmul_rn(drj, y);
+          const float auxa = (float)__dmul_rn(__fma_rn(2.0, rspd, ars1), iars2);
+          const float auxb = (float)__dsub_rn(edge, rspd);
+          const float s3 = mu(mu(auxa, auxb), auxb);
+          sw = sw_out ? s3 : ad(1.0f, -s3);
+          dsw = mu(mu(sgn, mu(2.0f * auxb, fm(auxb, iars2f, -auxa))), (float)y);
           if (EN) {
             const double auxbd = edge - rspd;
             const double s3d = (ars1 + 2.0 * rspd) * iars2 * auxbd * auxbd;
@@ -493,317 +466,441 @@ __global__ void __launch_bounds__(WPB * 32, MINB) k_pair(const PairArgs A) {
           }
         }
       }
-      // the j atoms to evaluate: all, or under lskip_ewald those with LJ --
-      // and all atoms of a switched pair, which take the S'V term by mass
-      // fraction whether they have LJ or not
-      unsigned bm = 0u;
-      if (inb) {
-        bm = (1u << (mj.y & 0xff)) - 1u;
-        if (ljonly && dsw == 0.f) bm &= (unsigned)(mj.y >> 16);
-      }
-      const int na = __popc(bm);
-      int sc = na;  // inclusive scan of the slot counts over the segment
-#pragma unroll
-      for (int o = 1; o < LPG; o <<= 1) {
-        const int v = __shfl_up_sync(FULL, sc, o);
-        if (sl >= o) sc += v;
-      }
-      const int tot = __shfl_sync(FULL, sc, seg0 + LPG - 1);
-      const unsigned bq = segbits(__ballot_sync(FULL, na > 0));
-      if (na > 0) {
-        const int e = (qh + qn + __popc(bq & below)) & (QE - 1);
-        s_edc[q][e] = make_float4((float)cx, (float)cy, (float)cz, sw);
-        s_edsw[q][e] = dsw;
-        s_emeta[q][e] = mj;
-        s_emsk[q][e] = msk;
-        if constexpr (EN) {
-          s_ecd[q][e] = make_double4(cx, cy, cz, swd);
-          if (A.stress)  // j sits at its image xpg_j + img: its virial arm gains co.img
-            s_eimg[q][e] = make_float4((float)(A.c11 * imx + A.c12 * imy + A.c13 * imz),
-                                       (float)(A.c22 * imy + A.c23 * imz), (float)(A.c33 * imz), 0.f);
+      // Entries with alchemical or fixed-mass atoms are queued a j atom at a
+      // time (V and the S'V term are sums over the pairs): their pairs are
+      // evaluated one after another, with FP64 work terms along a schedule,
+      // and a lane with a whole entry of them would hold up its warp.
+      const bool special = ALCH && ((mi.y | mj.y) & GM_SPECIAL);
+      bool more = true;
+      for (int part = 0; more; part++) {
+        const Bits push = special ? bits & (COLS << part) : (part ? (Bits)0 : bits);
+        const Bits rest = special ? bits & ~(Bits)(COLS * ((2u << part) - 1u)) : (Bits)0;
+        more = ALCH && __any_sync(FULL, rest != 0);
+        const unsigned bq = segbits(__ballot_sync(FULL, push != 0));
+        if (push != 0) {
+          const int e = (qh + qn + __popc(bq & below)) & (QE - 1);
+          s_edc[q][e] = make_float4((float)cx, (float)cy, (float)cz, sw);
+          s_emeta[q][e] = make_int4(mj.x, mj.y, mj.z, mj.w);
+          s_edsw[q][e] = dsw;
+          s_ebits[q][e] = push;
+          if constexpr (EN) {
+            s_ecd[q][e] = make_double4(cx, cy, cz, swd);
+            if (A.stress)  // j sits at its image xpg_j + img: its virial arm gains co.img
+              s_eimg[q][e] = make_double4(A.c11 * imx + A.c12 * imy + A.c13 * imz, A.c22 * imy + A.c23 * imz,
+                                          A.c33 * imz, 0.0);
+          }
         }
-        const int ps = sh + sn + sc - na;
-        unsigned bb = bm;
-        for (int t = 0; t < na; t++) {
-          const int b = __ffs(bb) - 1;
-          bb &= bb - 1u;
-          s_slot[q][(ps + t) & (QS - 1)] = slot_pack(e, t, b, na);
-        }
-      }
-      qn += __popc(bq);
-      sn += tot;
-      __syncwarp();
+        qn += __popc(bq);
+        __syncwarp();
 
-      // ---- phase 2: passes over whole entries, a lane per j atom
-      const bool last = base + LPG >= m;
-      for (;;) {
-        const bool want = sn >= LPG || (last && sn > 0);
-        if (!__any_sync(FULL, want)) break;
-        int L = 0;
-        if (want) {
-          L = sn;
-          if (sn > LPG) L = LPG - (((int)s_slot[q][(sh + LPG) & (QS - 1)] >> 6) & 7);
-          else if (sn == LPG) L = LPG;
-        }
-        const bool act = sl < L;
-        const unsigned r = act ? (unsigned)s_slot[q][(sh + sl) & (QS - 1)] : 0u;
-        const int e = r & 63, t = (r >> 6) & 7, b = (r >> 9) & 7, nsl = ((r >> 12) & 7) + 1;
-        float fbx = 0.f, fby = 0.f, fbz = 0.f, vpart = 0.f;
-        float4 dcs = make_float4(0.f, 0.f, 0.f, 1.f);
-        float dswe = 0.f;
-        int jat = 0, typej = 0;
-        if (act) {
-          dcs = s_edc[q][e];
-          dswe = s_edsw[q][e];
-          const int2 me = s_emeta[q][e];
-          const unsigned long long mskb = s_emsk[q][e] >> b;
-          jat = me.x + b;
-          typej = (me.y >> 8) & 0xff;
-          const float4 ob = A.aoff[jat];
-          const int tb = A.atype[jat];
-          const double qbd = EN ? A.qd[jat] : 0.0;
-          const int fjb = (VAR != VAR_STD) ? (int)A.vflag[jat] : 0;
-          const float2 sfb = ALCH ? A.soft[jat] : make_float2(0.f, 0.f);
-          const float bx = dcs.x - ob.x, by = dcs.y - ob.y, bz = dcs.z - ob.z;
-          double4 cd = make_double4(0.0, 0.0, 0.0, 1.0);
-          if (EN) cd = s_ecd[q][e];
-          double pconf = 0.0, pcoul = 0.0, px0 = 0.0, px1 = 0.0, px2 = 0.0;
+        // ---- phase 2: a lane per queued entry
+        const bool last = base + LPG >= m && !more;
+        for (;;) {
+          const int take = qn >= LPG ? LPG : (last ? qn : 0);
+          if (!__any_sync(FULL, take > 0)) break;
+          if (sl < take) {
+            const int e = (qh + sl) & (QE - 1);
+            const float4 dcs = s_edc[q][e];
+            const int4 me = s_emeta[q][e];
+            const Bits pb = s_ebits[q][e];
+            const int jf = me.x, nj = me.y & 15;
+            const float dswe = s_edsw[q][e];
+            double4 cd = make_double4(0.0, 0.0, 0.0, 1.0);
+            if (EN) cd = s_ecd[q][e];
+            float fi[MG][3], fj[MG <= 4 ? MG : 1][3];
+            double gjx = 0.0, gjy = 0.0, gjz = 0.0;  // the j group's force (image virial)
 #pragma unroll
-          for (int a = 0; a < MG; a++) {
-            if (a >= ni) break;
-            if ((mskb >> (a * 8)) & 1ull) continue;
-            if (ljonly && !((ljmi >> a) & 1)) continue;
-            const float4 ai = s_ai[q][a];  // a broadcast read
-            const float rx = ai.x + bx, ry = ai.y + by, rz = ai.z + bz;
-            float qf = 0.f, conf = 0.f, coul = 0.f;
-            bool ljon = false;
-            int tal = 0;
-            if constexpr (ALCH) {
-              // src/force_alchemy.f:412-451: exclusions and fixed-mass pairs
-              // are always skipped; no LJ and no Coulomb skips the pair
-              const int fia = s_fi[q][a];
-              if (fia & fjb & VF_MINF) continue;
-              const float2 sa = s_sf[q][a];
-              const float eps4 = sa.y * sfb.y;
-              if (eps4 < 1e-12f && A.lskip && A.ewald) continue;
-              npairs++;
-              tal = (fia >> VF_SSHIFT) + (fjb >> VF_SSHIFT) - 4;
-              alch_pair_f32(A, s_af, s_afq, rx * rx + ry * ry + rz * rz, tal, sa.x, sfb.x, eps4, ai.w * ob.w, &qf, &conf,
-                            &coul);
-              if constexpr (VAR == VAR_ALCHW) {
-                if (tal != 6) {  // 6: two normal atoms
+            for (int a = 0; a < MG; a++) fi[a][0] = fi[a][1] = fi[a][2] = 0.f;
+#pragma unroll
+            for (int b = 0; b < (MG <= 4 ? MG : 1); b++) fj[b][0] = fj[b][1] = fj[b][2] = 0.f;
+            float V = 0.f;
+            double pconf = 0.0, pcoul = 0.0, px0 = 0.0, px1 = 0.0, px2 = 0.0;
+            // the straight path: every pair of the two groups without a branch,
+            // so that the pairs' chains of dependent instructions overlap; pairs
+            // that are not to be evaluated take part at distance 1 with
+            // coefficients 0.  Three pairs share one test for LJ (in water only
+            // the oxygens have it).  Not for pairs of LJ alone (one in nine of
+            // water's) nor for groups with alchemical or fixed-mass atoms.
+            const bool straight = MG <= 4 && !A.lskip && !(ALCH && ((mi.y | me.y) & GM_SPECIAL));
+            if constexpr (MG <= 4) {
+              if (straight) {
+                npairs += __popc((unsigned)pb);
+                float4 ob[MG];
+#pragma unroll
+                for (int b = 0; b < MG; b++)
+                  ob[b] = b < nj ? A.aoff[jf + b] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int b = 0; b < MG; b++) {
+                  const float bx = ad(dcs.x, -ob[b].x), by = ad(dcs.y, -ob[b].y), bz = ad(dcs.z, -ob[b].z);
+                  float rx[MG], ry[MG], rz[MG], rsqi[MG], qf[MG], u[MG];
+#pragma unroll
+                  for (int a = 0; a < MG; a++) {
+                    const float4 ai = s_ai[q][a];  // a broadcast read
+                    const bool on = ((unsigned)pb >> (a * 8 + b)) & 1u;
+                    rx[a] = ad(ai.x, bx);
+                    ry[a] = ad(ai.y, by);
+                    rz[a] = ad(ai.z, bz);
+                    float r2 = fm(rz[a], rz[a], fm(ry[a], ry[a], mu(rx[a], rx[a])));
+                    r2 = on ? r2 : 1.f;
+                    const float qq = on ? mu(ai.w, ob[b].w) : 0.f;
+                    // 1/r from the hardware reciprocal square root, exp from ex2
+                    // and an approximate reciprocal: a few ulp, far below the
+                    // pair's FP32 rounding budget
+                    const float rinv = rsqrtf(r2);
+                    rsqi[a] = mu(rinv, rinv);
+                    const float qt = __fdividef(1.0f, fm(asqp, mu(r2, rinv), 1.0f));
+                    const float qe = mu(qq, ex2f(mu(a2l2, r2)));
+                    const float poly = fm(fm(fm(fm(AS_A5, qt, AS_A4), qt, AS_A3), qt, AS_A2), qt, AS_A1);
+                    u[a] = mu(mu(mu(poly, qt), qe), rinv);
+                    qf[a] = fm(twa, qe, u[a]);
+                  }
+                  if ((me.y >> (8 + b)) & 1) {  // the j atom has LJ
+                    const int tb = b < 2 ? (me.z >> (16 * b)) & 0xffff : (me.w >> (16 * (b - 2))) & 0xffff;
+#pragma unroll
+                    for (int a = 0; a < MG; a++) {
+                      const bool on = ((unsigned)pb >> (a * 8 + b)) & 1u;
+                      float u12, u6;
+                      if constexpr (ALCH) {  // two normal atoms: full strength, force_alchemy's sigma and epsilon
+                        const float2 sa = s_sf[q][a], sb = A.soft[jf + b];
+                        const float eps4 = on && sa.y * sb.y > 1e-12f ? sa.y * sb.y : 0.f;
+                        const float sig = A.at.opls ? 2.f * sqrtf(mu(sa.x, sb.x)) : ad(sa.x, sb.x);
+                        const float s2 = mu(mu(sig, sig), rsqi[a]);
+                        const float x = mu(mu(s2, s2), s2);
+                        u6 = mu(eps4, x);
+                        u12 = mu(u6, x);
+                      } else {
+                        const float2 L = __ldg(lj + s_ti[q][a] + tb);
+                        const float r6 = on ? mu(mu(rsqi[a], rsqi[a]), rsqi[a]) : 0.f;
+                        u6 = mu(L.y, r6);
+                        u12 = mu(mu(L.x, r6), r6);
+                      }
+                      qf[a] = fm(12.0f, u12, fm(-6.0f, u6, qf[a]));
+                      u[a] = ad(u[a], ad(u12, -u6));
+                    }
+                  }
+                  float fbx = 0.f, fby = 0.f, fbz = 0.f;
+#pragma unroll
+                  for (int a = 0; a < MG; a++) {
+                    // force_rem (src/force_REM.f:491-495,634-678): selected pairs
+                    // scale their force and their share of the S'V sum
+                    float w = dcs.w;
+                    bool sel = false;
+                    if constexpr (VAR == VAR_REM) {
+                      const bool ra = (mi.y >> (GM_REM + a)) & 1, rb = (me.y >> (GM_REM + b)) & 1;
+                      sel = A.rem_kind == 0 ? (ra || rb) : (A.rem_kind == 1 ? (ra && rb) : (ra != rb));
+                      w = sel ? mu(w, remf) : w;
+                      V = sel ? fm(u[a], remf, V) : ad(V, u[a]);
+                    } else {
+                      V = ad(V, u[a]);
+                    }
+                    const float f = mu(mu(qf[a], rsqi[a]), w);
+                    fi[a][0] = fm(f, rx[a], fi[a][0]);
+                    fi[a][1] = fm(f, ry[a], fi[a][1]);
+                    fi[a][2] = fm(f, rz[a], fi[a][2]);
+                    fbx = fm(-f, rx[a], fbx);
+                    fby = fm(-f, ry[a], fby);
+                    fbz = fm(-f, rz[a], fbz);
+                  }
+                  fj[b][0] = fbx;
+                  fj[b][1] = fby;
+                  fj[b][2] = fbz;
+                  if (EN) {
+                    gjx += fbx;
+                    gjy += fby;
+                    gjz += fbz;
+                  }
+                }
+              }
+            }
+            if (!straight) {
+              if (!ljonly && !ALCH) npairs += MG > 4 ? __popcll(pb) : __popc((unsigned)pb);
+#pragma unroll 1
+              for (int b = 0; b < MG; b++) {
+                const Bits col = (pb >> b) & COLS;  // the i atoms of this j atom's pairs
+                if (!col) continue;
+                float fbx = 0.f, fby = 0.f, fbz = 0.f;
+                const int jat = jf + b;
+                const float4 ob = A.aoff[jat];
+                const int tb = A.atype[jat];
+                const int fjb = (VAR != VAR_STD) ? (int)A.vflag[jat] : 0;
+                const float2 sfb = ALCH ? A.soft[jat] : make_float2(0.f, 0.f);
+                const float bx = ad(dcs.x, -ob.x), by = ad(dcs.y, -ob.y), bz = ad(dcs.z, -ob.z);
+#pragma unroll
+                for (int a = 0; a < MG; a++) {
+                  if (!((col >> (a * 8)) & 1)) continue;
+                  const float4 ai = s_ai[q][a];  // a broadcast read
+                  const float rx = ad(ai.x, bx), ry = ad(ai.y, by), rz = ad(ai.z, bz);
+                  const float r2 = fm(rz, rz, fm(ry, ry, mu(rx, rx)));
+                  float qf = 0.f, conf = 0.f, coul = 0.f;
+                  if constexpr (ALCH) {
+                    // src/force_alchemy.f:412-451: exclusions and fixed-mass pairs
+                    // are always skipped; no LJ and no Coulomb skips the pair
+                    const int fia = s_fi[q][a];
+                    if (fia & fjb & VF_MINF) continue;
+                    const float2 sa = s_sf[q][a];
+                    const float eps4 = sa.y * sfb.y;
+                    if (eps4 < 1e-12f && ljonly) continue;
+                    npairs++;
+                    alch_pair_f32(A, s_af, s_afq, r2, (fia >> VF_SSHIFT) + (fjb >> VF_SSHIFT) - 4, sa.x, sfb.x, eps4,
+                                  ai.w * ob.w, &qf, &conf, &coul);
+                  } else {
+                    const float2 Lp = __ldg(lj + s_ti[q][a] + tb);
+                    const bool ljon = Lp.y != 0.f;
+                    if (ljonly) {  // src/force.f:416-417
+                      if (!ljon) continue;
+                      npairs++;
+                    }
+                    const float rinv = rsqrtf(r2);
+                    const float rsqi = mu(rinv, rinv);
+                    if (ljon) {
+                      const float r6 = mu(mu(rsqi, rsqi), rsqi);
+                      const float u6 = mu(Lp.y, r6), u12 = mu(mu(Lp.x, r6), r6);
+                      qf = fm(12.0f, u12, mu(-6.0f, u6));
+                      conf = ad(u12, -u6);
+                    }
+                    if (!A.lskip) {
+                      const float qt = __fdividef(1.0f, fm(asqp, mu(r2, rinv), 1.0f));
+                      const float qe = mu(mu(ai.w, ob.w), ex2f(mu(a2l2, r2)));
+                      const float poly = fm(fm(fm(fm(AS_A5, qt, AS_A4), qt, AS_A3), qt, AS_A2), qt, AS_A1);
+                      coul = mu(mu(mu(poly, qt), qe), rinv);
+                      qf = ad(qf, fm(twa, qe, coul));
+                    } else if (!A.ewald) {
+                      coul = mu(mu(ai.w, ob.w), rinv);
+                      qf = ad(qf, coul);
+                    }
+                    qf = mu(qf, rsqi);
+                  }
+                  // force_rem (src/force_REM.f:491-495,634-678): selected pairs scale
+                  // their force and their share of the S'V sum
+                  const bool sel = (VAR == VAR_REM) && seg_sel(A.rem_kind, s_fi[q][a], fjb);
+                  V = sel ? fm(ad(conf, coul), remf, V) : ad(V, ad(conf, coul));
+                  qf = mu(qf, dcs.w);
+                  if (sel) qf = mu(qf, remf);
+                  fi[a][0] = fm(qf, rx, fi[a][0]);
+                  fi[a][1] = fm(qf, ry, fi[a][1]);
+                  fi[a][2] = fm(qf, rz, fi[a][2]);
+                  fbx = fm(-qf, rx, fbx);
+                  fby = fm(-qf, ry, fby);
+                  fbz = fm(-qf, rz, fbz);
+                }
+                if constexpr (MG <= 4) {
+#pragma unroll
+                  for (int c = 0; c < MG; c++)
+                    if (c == b) {
+                      fj[c][0] = fbx;
+                      fj[c][1] = fby;
+                      fj[c][2] = fbz;
+                    }
+                } else {
+                  fix_add(A.ffix + jat, fbx);
+                  fix_add(A.ffix + A.natom + jat, fby);
+                  fix_add(A.ffix + 2 * A.natom + jat, fbz);
+                }
+                if (EN) {
+                  gjx += fbx;
+                  gjy += fby;
+                  gjz += fbz;
+                }
+              }
+            }
+            // along a schedule, force_alchemy's dwrk of an entry with alchemical
+            // atoms (one j atom): U(lambda) - U(lambda0) of its pairs
+            if constexpr (VAR == VAR_ALCHW) {
+              if ((mi.y | me.y) & GM_SPECIAL) {
+                const int b = MG > 4 ? (__ffsll((long long)pb) - 1) & 7 : (__ffs((int)pb) - 1) & 7;
+                const int jat = jf + b;
+                const float4 ob = A.aoff[jat];
+                const float bx = ad(dcs.x, -ob.x), by = ad(dcs.y, -ob.y), bz = ad(dcs.z, -ob.z);
+                const int fjb = A.vflag[jat];
+                const double2 sj = A.softd[jat];
+                const double qj = A.qd[jat];
+                const float yj = A.soft[jat].y;
+#pragma unroll
+                for (int a = 0; a < MG; a++) {
+                  if (!((pb >> (a * 8 + b)) & 1)) continue;
+                  const int fia = s_fi[q][a], tal = (fia >> VF_SSHIFT) + (fjb >> VF_SSHIFT) - 4;
+                  if (tal == 6 || (fia & fjb & VF_MINF)) continue;  // 6: two normal atoms
+                  if (s_sf[q][a].y * yj < 1e-12f && ljonly) continue;
+                  const float4 ai = s_ai[q][a];
                   double cdd, qdd, c0, q0, du;
-                  alch_energy_fp64(A, (double)rx, (double)ry, (double)rz, A.softd[ifirst + a], A.softd[jat],
-                                   A.qd[ifirst + a] * A.qd[jat], tal, &cdd, &qdd, &c0, &q0, &du);
+                  alch_energy_fp64(A, (double)ad(ai.x, bx), (double)ad(ai.y, by), (double)ad(ai.z, bz),
+                                   A.softd[ifirst + a], sj, A.qd[ifirst + a] * qj, tal, &cdd, &qdd, &c0, &q0, &du);
                   wk += ((cdd + qdd) - (c0 + q0)) * (double)dcs.w;
                 }
               }
-            } else {
-              const float2 Lp = lj[s_ti[q][a] + tb];
-              ljon = Lp.y != 0.f;
-              if (A.lskip && !ljon && A.ewald) continue;  // src/force.f:416-417
-              npairs++;
-              const float r2 = rx * rx + ry * ry + rz * rz;
-              // 1/r from the hardware reciprocal square root, exp from ex2 and
-              // an approximate reciprocal: a few ulp, far below the pair's FP32
-              // rounding budget, and a fraction of the IEEE sequences' cost
-              const float rinv = rsqrtf(r2);
-              const float rsqi = rinv * rinv;
-              if (ljon) {
-                const float r6 = rsqi * rsqi * rsqi;
-                const float r12 = r6 * r6;
-                qf = (12.0f * Lp.x * r12 - 6.0f * Lp.y * r6) * rsqi;
-                conf = Lp.x * r12 - Lp.y * r6;
-              }
-              if (!A.lskip) {
-                const float rsp = r2 * rinv;
-                const float ar = A.alphal * rsp;
-                const float qt = __fdividef(1.0f, 1.0f + AS_QP * ar);
-                const float ex = __expf(-ar * ar);
-                const float erfcst = ((((AS_A5 * qt + AS_A4) * qt + AS_A3) * qt + AS_A2) * qt + AS_A1) * qt * ex;
-                const float qq = ai.w * ob.w;
-                coul = qq * erfcst * rinv;
-                qf += qq * (erfcst + A.twrtpi * ar * ex) * rsqi * rinv;
-              } else if (!A.ewald) {
-                coul = ai.w * ob.w * rinv;
-                qf += coul * rsqi;
+            }
+            // the FP64 pair energies: one rolled loop over the entry's pairs
+            if constexpr (EN) {
+#pragma unroll 1
+              for (Bits rest = pb; rest; rest &= rest - 1) {
+                const int bit = MG > 4 ? __ffsll((long long)rest) - 1 : __ffs((int)rest) - 1;
+                const int a = bit >> 3, jat = jf + (bit & 7);
+                const float4 ai = s_ai[q][a], ob = A.aoff[jat];
+                const double erx = cd.x + ((double)ai.x - (double)ob.x);
+                const double ery = cd.y + ((double)ai.y - (double)ob.y);
+                const double erz = cd.z + ((double)ai.z - (double)ob.z);
+                double cdd, qdd;
+                if constexpr (ALCH) {
+                  const int fia = s_fi[q][a], fjb = A.vflag[jat];
+                  if (fia & fjb & VF_MINF) continue;
+                  if (s_sf[q][a].y * A.soft[jat].y < 1e-12f && ljonly) continue;
+                  double c0, q0, du;
+                  alch_energy_fp64(A, erx, ery, erz, A.softd[ifirst + a], A.softd[jat], s_qd[q][a] * A.qd[jat],
+                                   (fia >> VF_SSHIFT) + (fjb >> VF_SSHIFT) - 4, &cdd, &qdd, &c0, &q0, &du);
+                  px0 += c0;
+                  px1 += q0;
+                  px2 += du;
+                } else {
+                  const double2 L = A.ljd[s_ti[q][a] + A.atype[jat]];
+                  if (ljonly && L.y == 0.0) continue;
+                  pair_energy_fp64(A, erx, ery, erz, L, L.y != 0.0, s_qd[q][a] * A.qd[jat], &cdd, &qdd);
+                  if (VAR == VAR_REM && seg_sel(A.rem_kind, s_fi[q][a], A.vflag[jat])) px0 += cdd + qdd;  // seg_ene
+                }
+                pconf += cdd;
+                pcoul += qdd;
               }
             }
-            // force_rem (src/force_REM.f:491-495,634-678): selected pairs scale
-            // their force and their share of the S'V sum
-            const bool sel = (VAR == VAR_REM) && seg_sel(A.rem_kind, s_fi[q][a], fjb);
-            vpart += sel ? (conf + coul) * remf : conf + coul;
-            qf *= dcs.w;
-            if (sel) qf *= remf;
-            if (EN) {
-              const double erx = cd.x + ((double)ai.x - (double)ob.x);
-              const double ery = cd.y + ((double)ai.y - (double)ob.y);
-              const double erz = cd.z + ((double)ai.z - (double)ob.z);
-              double cdd, qdd;
-              if constexpr (ALCH) {
-                double c0, q0, du;
-                alch_energy_fp64(A, erx, ery, erz, A.softd[ifirst + a], A.softd[jat], s_qd[q][a] * qbd, tal, &cdd,
-                                 &qdd, &c0, &q0, &du);
-                px0 += c0;
-                px1 += q0;
-                px2 += du;
-              } else {
-                pair_energy_fp64(A, erx, ery, erz, A.ljd[s_ti[q][a] + tb], ljon, s_qd[q][a] * qbd, &cdd, &qdd);
-                if (sel) px0 += cdd + qdd;  // seg_ene
-              }
-              pconf += cdd;
-              pcoul += qdd;
-            }
-            const float fx = qf * rx, fy = qf * ry, fz = qf * rz;
-            fiq[a][0] += to_fix(fx);
-            fiq[a][1] += to_fix(fy);
-            fiq[a][2] += to_fix(fz);
-            fbx -= fx;
-            fby -= fy;
-            fbz -= fz;
-          }
-          if constexpr (EN) {
-            const int tt = typei + typej - 2;  // 0 slt-slt, 1 slt-slv, 2 slv-slv
-            pconf *= cd.w;
-            pcoul *= cd.w;
-            if (tt == 0) {
-              ec0 += pconf;
-              eq0 += pcoul;
-            } else if (tt == 1) {
-              ec1 += pconf;
-              eq1 += pcoul;
-            } else {
-              ec2 += pconf;
-              eq2 += pcoul;
-            }
-            ex0 += px0 * cd.w;
-            ex1 += px1 * cd.w;
-            ex2 += px2 * cd.w;
-          }
-        }
-        // S'(R) V term of switched entries (src/force.f:754-817): V summed
-        // over the entry's lanes, X = -dS/dR / R V R_vec distributed by mass
-        // fraction, on the j atoms here and on the i atoms at the end of the row
-        if (__any_sync(FULL, dswe != 0.f)) {
-          float v = vpart;
+            // S'(R) V term of a switched entry (src/force.f:754-817): X = -dS/dR / R
+            // V R_vec distributed by mass fraction over both groups' atoms
+            if (dswe != 0.f) {
+              const float sv = mu(-dswe, V);
+              const float sx = mu(sv, dcs.x), sy = mu(sv, dcs.y), sz = mu(sv, dcs.z);
+              if constexpr (MG <= 4) {
 #pragma unroll
-          for (int o = 1; o < MG; o <<= 1) {
-            const float w = __shfl_down_sync(FULL, v, o);
-            if (t + o < nsl) v += w;
-          }
-          const float V = __shfl_sync(FULL, v, (lane - t) & 31);
-          if (act && dswe != 0.f) {
-            const float sx = -dswe * V * dcs.x, sy = -dswe * V * dcs.y, sz = -dswe * V * dcs.z;
-            const float pm = A.apm[jat];
-            fbx -= pm * sx;
-            fby -= pm * sy;
-            fbz -= pm * sz;
-            if (t == 0) {  // the i atoms' share, by mass fraction
+                for (int b = 0; b < MG; b++) {
+                  const float pm = b < nj ? A.apm[jf + b] : 0.f;
+                  fj[b][0] = fm(-pm, sx, fj[b][0]);
+                  fj[b][1] = fm(-pm, sy, fj[b][1]);
+                  fj[b][2] = fm(-pm, sz, fj[b][2]);
+                }
+              } else {
+                for (int b = 0; b < nj; b++) {
+                  const float pm = A.apm[jf + b];
+                  fix_add(A.ffix + jf + b, -pm * sx);
+                  fix_add(A.ffix + A.natom + jf + b, -pm * sy);
+                  fix_add(A.ffix + 2 * A.natom + jf + b, -pm * sz);
+                }
+              }
 #pragma unroll
               for (int a = 0; a < MG; a++) {
-                if (a >= ni) break;
                 const float pmi = s_pm[q][a];
-                fiq[a][0] += to_fix(pmi * sx);
-                fiq[a][1] += to_fix(pmi * sy);
-                fiq[a][2] += to_fix(pmi * sz);
+                fi[a][0] = fm(pmi, sx, fi[a][0]);
+                fi[a][1] = fm(pmi, sy, fi[a][1]);
+                fi[a][2] = fm(pmi, sz, fi[a][2]);
+              }
+              if (EN) {
+                gjx -= sx;
+                gjy -= sy;
+                gjz -= sz;
+              }
+            }
+            if constexpr (MG <= 4) {
+#pragma unroll
+              for (int b = 0; b < MG; b++) {  // (zero beyond the group's atoms)
+                fix_add(A.ffix + jf + b, fj[b][0]);
+                fix_add(A.ffix + A.natom + jf + b, fj[b][1]);
+                fix_add(A.ffix + 2 * A.natom + jf + b, fj[b][2]);
+              }
+            }
+#pragma unroll
+            for (int c = 0; c < 3 * MG; c++) {
+              const long long add = to_fix(fi[c / 3][c % 3]);
+              s_fiq[c][threadIdx.x] = started ? s_fiq[c][threadIdx.x] + add : add;
+            }
+            if constexpr (EN) {
+              const int tt = typei + ((me.y >> 4) & 15) - 2;  // 0 slt-slt, 1 slt-slv, 2 slv-slv
+              pconf *= cd.w;
+              pcoul *= cd.w;
+              if (tt == 0) {
+                ec0 += pconf;
+                eq0 += pcoul;
+              } else if (tt == 1) {
+                ec1 += pconf;
+                eq1 += pcoul;
+              } else {
+                ec2 += pconf;
+                eq2 += pcoul;
+              }
+              ex0 += px0 * cd.w;
+              ex1 += px1 * cd.w;
+              ex2 += px2 * cd.w;
+              if (A.stress) {
+                const double4 im = s_eimg[q][e];
+                const double g3[3] = {gjx, gjy, gjz}, i3[3] = {im.x, im.y, im.z};
+#pragma unroll
+                for (int c = 0; c < 9; c++) vimg[c] += g3[c / 3] * i3[c % 3];
               }
             }
           }
-        }
-        if (act) {
-          fix_add(A.ffix + jat, fbx);
-          fix_add(A.ffix + A.natom + jat, fby);
-          fix_add(A.ffix + 2 * A.natom + jat, fbz);
-        }
-        if (EN && A.stress) {
-          if (act) {
-            const float4 im = s_eimg[q][e];
-            vimg[0] += fbx * im.x;
-            vimg[1] += fbx * im.y;
-            vimg[2] += fbx * im.z;
-            vimg[3] += fby * im.x;
-            vimg[4] += fby * im.y;
-            vimg[5] += fby * im.z;
-            vimg[6] += fbz * im.x;
-            vimg[7] += fbz * im.y;
-            vimg[8] += fbz * im.z;
+          if (take > 0 && take < LPG && !started && sl >= take) {
+#pragma unroll
+            for (int c = 0; c < 3 * MG; c++) s_fiq[c][threadIdx.x] = 0ll;
           }
-          flush_vimg();
+          started = started || take > 0;
+          qh += take;
+          qn -= take;
+          __syncwarp();
         }
-        const int ne = __popc(segbits(__ballot_sync(FULL, act && t == 0)));
-        sh += L;
-        sn -= L;
-        qh += ne;
-        qn -= ne;
-        __syncwarp();
       }
     }
     if (A.next_on && sl == 0 && gvalid) {
       A.cnt_out[i] = nout;
       nkept += (unsigned)nout;
     }
-    if (A.forces_on) {
-      // i atoms: the fixed-point sums of the segment's lanes by one
-      // reduce-scatter; the lane holding component c of atom a adds it
-      constexpr int P = 3 * MG <= 16 ? 16 : 32;
-      long long v[P];
-#pragma unroll
-      for (int a = 0; a < MG; a++) {
-        v[3 * a] = fiq[a][0];
-        v[3 * a + 1] = fiq[a][1];
-        v[3 * a + 2] = fiq[a][2];
-      }
-#pragma unroll
-      for (int k = 3 * MG; k < P; k++) v[k] = 0ll;
-      const long long tot_v = reduce_scatter<LPG, P>(v, sl);
-      const int idx = rs_index<LPG, P>(sl);
-      const bool owner = (LPG / P <= 1) || (sl % (LPG / P)) == 0;  // one lane per value
-      if (gvalid && m > 0 && owner && idx < 3 * ni && tot_v != 0)
-        atomicAdd(A.ffix + (idx % 3) * A.natom + ifirst + idx / 3, (unsigned long long)tot_v);
+    // i atoms: a lane sums one value over the row's lanes (of a whole-warp row, half
+    // of the lanes each) and adds it
+    constexpr int PARTS = (LPG == 32 && 3 * MG <= 16) ? 2 : 1;
+    const int val = sl % (LPG / PARTS), part = sl / (LPG / PARTS);
+    long long sum = 0ll;
+    if (started && val < 3 * ni) {
+      const long long* src = &s_fiq[val][warp * 32 + seg0 + part * (LPG / PARTS)];
+#pragma unroll 8
+      for (int k = 0; k < LPG / PARTS; k++) sum += src[k];
     }
-    __syncwarp();
+    if (PARTS == 2) sum += __shfl_xor_sync(FULL, sum, 16);
+    if (part == 0 && sum != 0ll)
+      atomicAdd(A.ffix + (val % 3) * A.natom + ifirst + val / 3, (unsigned long long)sum);
   }
   {
-    // work counters, one atomic per warp
-    unsigned s0 = nscan, s1 = nkept, s2 = npairs;
+    // work counters: one atomic per block and counter, over WCNT_SLOTS copies
+    // (a single copy's atomics of a launch wait for one another at the L2)
+    nscan = __reduce_add_sync(FULL, nscan);
+    nkept = __reduce_add_sync(FULL, nkept);
+    npairs = __reduce_add_sync(FULL, npairs);
+    if (lane < 3) s_cnt[warp][lane] = lane == 0 ? nscan : (lane == 1 ? nkept : npairs);
+  }
+  // energies and the image virial: the EN build only (a stress request
+  // selects it, pair_launch)
+  constexpr int NV = (VAR != VAR_STD) ? 18 : 15;
+  if constexpr (EN) {
+    const double vals[18] = {ec0, ec1, ec2, eq0, eq1, eq2, vimg[0], vimg[1], vimg[2],
+                             vimg[3], vimg[4], vimg[5], vimg[6], vimg[7], vimg[8], ex0, ex1, ex2};
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      s0 += __shfl_xor_sync(FULL, s0, o);
-      s1 += __shfl_xor_sync(FULL, s1, o);
-      s2 += __shfl_xor_sync(FULL, s2, o);
-    }
-    if (lane == 0) {
-      if (s0) atomicAdd(A.wcnt + 0, (unsigned long long)s0);
-      if (s1) atomicAdd(A.wcnt + 1, (unsigned long long)s1);
-      if (s2) atomicAdd(A.wcnt + (A.lskip ? 3 : 2), (unsigned long long)s2);
+    for (int c = 0; c < NV; c++) {
+      const double sred = warp_sumd(vals[c]);
+      if (lane == 0) s_red[warp][c] = sred;
     }
   }
   if constexpr (VAR == VAR_ALCHW) {
     const double w = warp_sumd(wk);
     if (lane == 0 && w != 0.0) atomicAdd(A.dwrk, w);
   }
-  // energies and the image virial: the EN build only (a stress request
-  // selects it, pair_launch)
-  if (!EN || !A.forces_on) return;
-  // block reduction of energies and image virial
-  constexpr int NV = (VAR != VAR_STD && EN) ? 18 : 15;
-  double vals[18] = {ec0, ec1, ec2, eq0, eq1, eq2, 0, 0, 0, 0, 0, 0, 0, 0, 0, ex0, ex1, ex2};
-#pragma unroll
-  for (int c = 0; c < NV; c++) {
-    if (c >= 6 && c < 15) {
-      if (lane == 0) s_red[warp][c] = s_vimg[warp][c - 6];
-      continue;
-    }
-    const double sred = warp_sumd(vals[c]);
-    if (lane == 0) s_red[warp][c] = sred;
-  }
   __syncthreads();
-  if (threadIdx.x < NV) {
-    double sacc = 0;
-    for (int w = 0; w < WPB; w++) sacc += s_red[w][threadIdx.x];
-    // slots 0..14 = ACC_CONF..ACC_VIMG+8, then ACC_X..ACC_X+2
-    const int acc_slot = threadIdx.x < 15 ? (int)threadIdx.x : ACC_X + (int)threadIdx.x - 15;
-    if (sacc != 0.0) atomicAdd(A.acc + acc_slot, sacc);
+  if (threadIdx.x < 3) {
+    unsigned s = 0;
+#pragma unroll
+    for (int w = 0; w < WPB; w++) s += s_cnt[w][threadIdx.x];
+    const int slot = threadIdx.x < 2 ? (int)threadIdx.x : (A.lskip ? 3 : 2);
+    if (s) atomicAdd(A.wcnt + 4 * (blockIdx.x % WCNT_SLOTS) + slot, (unsigned long long)s);
+  }
+  if constexpr (EN) {
+    if (A.forces_on && threadIdx.x < NV) {
+      double sacc = 0;
+      for (int w = 0; w < WPB; w++) sacc += s_red[w][threadIdx.x];
+      // slots 0..14 = ACC_CONF..ACC_VIMG+8, then ACC_X..ACC_X+2
+      const int acc_slot = threadIdx.x < 15 ? (int)threadIdx.x : ACC_X + (int)threadIdx.x - 15;
+      if (sacc != 0.0) atomicAdd(A.acc + acc_slot, sacc);
+    }
   }
 }
 
@@ -890,7 +987,6 @@ __global__ void k_finalize(int N, const unsigned long long* __restrict__ ffix,
 }  // namespace
 
 int pair_launch(orac_gpu_ctx* ctx, const PairArgs& a, int maxg) {
-  const size_t smem = (size_t)(a.ntype * a.ntype <= LJ_SMEM_MAX ? a.ntype * a.ntype : 0) * sizeof(float2);
   if (maxg > ORAC_MAXG)
     return ctx_fail(ctx, ORAC_ERR_PARAM, "charge group of %d atoms exceeds %d", maxg, ORAC_MAXG);
   if (a.variant < VAR_STD || a.variant > VAR_ALCH) return ctx_fail(ctx, ORAC_ERR_PARAM, "variant %d", a.variant);
@@ -901,10 +997,9 @@ int pair_launch(orac_gpu_ctx* ctx, const PairArgs& a, int maxg) {
   // for the two small bounds
   const int mgk = maxg <= 3 ? 0 : (maxg <= 4 ? 1 : 2);
   const bool half = mgk < 2 && a.lpg == 16;
-  const int gpb = WPB * (half ? 2 : 1);  // groups per block
-  if (a.split != 1 && (a.split != 2 || half || a.next_on))
-    return ctx_fail(ctx, ORAC_ERR_PARAM, "row split %d with %s", a.split, a.next_on ? "a next-shell list" : "lpg 16");
-  int nb = (a.ngrp * a.split + gpb - 1) / gpb;
+  const int wpb = warps_per_block(mgk == 2 ? 8 : 4);
+  const int gpb = wpb * (half ? 2 : 1);  // groups per block
+  int nb = (a.ngrp + gpb - 1) / gpb;
   if (nb < 1) nb = 1;
   int slot = -1;
   if (int rc = prof_begin(ctx, &slot)) return rc;
@@ -914,23 +1009,25 @@ int pair_launch(orac_gpu_ctx* ctx, const PairArgs& a, int maxg) {
   switch ((((mgk * 4 + var) * 2 + (en ? 1 : 0)) * 2 + (half ? 1 : 0)) * 3 + occ) {
 #define ORAC_KP(MGK, MG, VAR, EN, LPG, OCC, MINB)                                               \
   case (((MGK * 4 + VAR) * 2 + (EN ? 1 : 0)) * 2 + (LPG == 16 ? 1 : 0)) * 3 + OCC:             \
-    orac_launch(k_pair<MG, EN, VAR, LPG, MINB>, nb, WPB * 32, smem, ctx->stream, a);            \
+    orac_launch(k_pair<MG, EN, VAR, LPG, MINB>, nb, wpb * 32, 0, ctx->stream, a);            \
     break;
 #define ORAC_KP_L(MGK, MG, VAR, LPG)       \
-  ORAC_KP(MGK, MG, VAR, false, LPG, 0, 5)  \
+  ORAC_KP(MGK, MG, VAR, false, LPG, 0, 5) \
   ORAC_KP(MGK, MG, VAR, false, LPG, 1, 6)  \
   ORAC_KP(MGK, MG, VAR, false, LPG, 2, 8)  \
   ORAC_KP(MGK, MG, VAR, true, LPG, 0, 1)
 #define ORAC_KP_V(MGK, MG, VAR) \
   ORAC_KP_L(MGK, MG, VAR, 32)   \
   ORAC_KP_L(MGK, MG, VAR, 16)
+// (the FP64 work terms of its alchemical rows are the launch's longest chain:
+// registers before occupancy)
 #define ORAC_KP_W(MGK, MG)                         \
-  ORAC_KP(MGK, MG, VAR_ALCHW, false, 32, 0, 5)     \
-  ORAC_KP(MGK, MG, VAR_ALCHW, false, 32, 1, 6)     \
-  ORAC_KP(MGK, MG, VAR_ALCHW, false, 32, 2, 8)     \
-  ORAC_KP(MGK, MG, VAR_ALCHW, false, 16, 0, 5)     \
-  ORAC_KP(MGK, MG, VAR_ALCHW, false, 16, 1, 6)     \
-  ORAC_KP(MGK, MG, VAR_ALCHW, false, 16, 2, 8)
+  ORAC_KP(MGK, MG, VAR_ALCHW, false, 32, 0, 3)     \
+  ORAC_KP(MGK, MG, VAR_ALCHW, false, 32, 1, 4)     \
+  ORAC_KP(MGK, MG, VAR_ALCHW, false, 32, 2, 5)     \
+  ORAC_KP(MGK, MG, VAR_ALCHW, false, 16, 0, 3)     \
+  ORAC_KP(MGK, MG, VAR_ALCHW, false, 16, 1, 4)     \
+  ORAC_KP(MGK, MG, VAR_ALCHW, false, 16, 2, 5)
     ORAC_KP_V(0, 3, VAR_STD)
     ORAC_KP_V(0, 3, VAR_REM)
     ORAC_KP_V(0, 3, VAR_ALCH)

@@ -17,7 +17,7 @@
 int tune_candidates(int maxg, std::vector<PairTune>* out) {
   out->clear();
   if (maxg > 4) {  // groups of up to 8 atoms: one build (a warp per group)
-    out->push_back({32, 32, 6});
+    out->push_back({32, 32, 5});
     return ORAC_OK;
   }
   const int lp[2] = {16, 32}, mb[3] = {5, 6, 8};
@@ -52,7 +52,7 @@ std::string tune_signature(const std::vector<orac_gpu_ctx*>& ctxs, const char* w
   }
   std::ostringstream s;
   s << dev << ";" << what << ";systems=" << ctxs.size() << ";atoms=" << atoms << ";max_atoms=" << amax
-    << ";maxg=" << maxg << ";variants=" << var;
+    << ";maxg=" << maxg << ";variants=" << var << ";entry";  // (choices of the lane-per-entry kernel)
   return s.str();
 }
 
@@ -95,9 +95,10 @@ int orac_gpu_set_pair_tuning(orac_gpu_ctx* ctx, int lpg_m, int lpg_lh, int minb)
 
 int orac_gpu_get_pair_tuning(orac_gpu_ctx* ctx, int* out3) {
   if (!ctx || !out3) return ORAC_ERR_PARAM;
-  out3[0] = ctx->tune_lpg_m ? ctx->tune_lpg_m : (ctx->shared_device ? 16 : 32);
-  out3[1] = ctx->tune_lpg_lh ? ctx->tune_lpg_lh : 32;
-  out3[2] = ctx->tune_minb ? ctx->tune_minb : (ctx->shared_device ? 8 : 6);
+  int minb = 0;
+  pair_config(ctx, &out3[0], &minb, true);
+  pair_config(ctx, &out3[1], &minb, false);
+  out3[2] = minb;
   return ORAC_OK;
 }
 

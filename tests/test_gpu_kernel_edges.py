@@ -1,0 +1,108 @@
+"""GPU kernels at the sizes where their tiles end, against the FP64 oracle:
+the pair kernel's rows (one group pair to several passes, groups of up to 3,
+4 and 8 atoms, half and whole warps a row) and the seam of the list's
+ownership rule, the plane FFT (odd axes, one x line left over, planes too
+large for shared memory) and the plan kept for calls that bring their own
+grid.  Tolerances as in the other parity tests: forces relative RMS <= 1e-5
+(FP32 pair and spline arithmetic), energies 1e-6 of the terms' magnitudes.
+"""
+import numpy as np
+import pytest
+
+import oracle
+from orac_b200 import systems
+
+pytestmark = pytest.mark.gpu
+
+
+def rel_rms(F, Fref):
+    return float(np.sqrt(((F - Fref) ** 2).sum() / max((Fref ** 2).sum(), 1e-300)))
+
+
+def small_shells():
+    return systems.Shells(rcutm=3.5, rtolm=0.3, rneim=0.4, rcutl=5.5, rtoll=0.3, rneil=0.4, rcuth=8.0, rtolh=0.3,
+                          rneih=0.6)
+
+
+@pytest.mark.parametrize("nwat", [2, 3, 4, 17, 64, 65])
+def test_rows_and_ownership_of_few_groups(nwat):
+    """All-pairs lists of 2 to 65 groups: rows of no entry to several passes,
+    and for even counts the pairs half the index circle apart."""
+    from orac_b200.engine import Engine
+
+    s = systems.water_box(nwat=nwat, box=18.8, lattice=5, nfft=(20, 20, 20))
+    s.ncell = None
+    s.shells = small_shells()
+    o, g = oracle.Oracle(s.copy()), Engine(s.copy())
+    o.update_lists()
+    g.update_lists()
+    for sh in "mlh":
+        Fr, uer, sr = o.shell(sh)
+        Fg, en, sg = g.shell(sh)
+        scale = np.abs(uer).sum() + 1e-300
+        # relative RMS; a shell without pairs has no forces on either side
+        assert np.sqrt(((Fg - Fr) ** 2).sum()) <= 1e-5 * np.sqrt((Fr ** 2).sum()), sh
+        assert np.abs(g.ue6(en) - uer).max() <= 1e-6 * scale
+        assert np.linalg.norm(sg - sr) <= 1e-5 * max(np.linalg.norm(sr), 1e-12)
+    g.close()
+
+
+@pytest.mark.parametrize("group_size", [1, 3, 4, 5, 8])
+@pytest.mark.parametrize("lanes", [(16, 16), (32, 32)])
+def test_group_sizes_and_lanes(group_size, lanes):
+    """Chains cut in groups of 1 to 8 atoms in water: each build of the pair
+    kernel, with exclusion masks on both sides of the ownership rule."""
+    from orac_b200.engine import Engine
+
+    s = systems.solvated_chains(2100, 31, group_size=group_size)
+    o, g = oracle.Oracle(s.copy()), Engine(s.copy())
+    g.set_pair_tuning(*lanes, 5)
+    o.update_lists()
+    g.update_lists()
+    for sh in "mlh":
+        Fr, uer, sr = o.shell(sh)
+        Fg, en, sg = g.shell(sh)
+        assert rel_rms(Fg, Fr) <= 1e-5
+        assert np.abs(g.ue6(en) - uer).max() <= 1e-6 * np.abs(uer).sum()
+        assert np.linalg.norm(sg - sr) <= 1e-5 * np.linalg.norm(sr)
+    g.close()
+
+
+@pytest.mark.parametrize("variant", ["std", "rem", "alchemy"])
+def test_forces_do_not_depend_on_energies_or_lanes(variant):
+    """The same forces bit for bit with and without energies and for every
+    launch configuration."""
+    import torch
+
+    from orac_b200.engine import Engine
+
+    s = systems.ligand_in_water(nlig=13, nwat=1000, box=31.3, nfft=(32, 32, 32))
+    s.ncell = (systems.linked_cells_for(31.3, s.shells),) * 3
+    got = {}
+    for cfg in ((16, 16, 5), (32, 32, 5), (16, 32, 6), (32, 16, 8)):
+        g = Engine(s.copy())
+        if variant == "rem":
+            g.set_rem((s.ss_alchemy == -2).astype(int), 0, 0.7)
+        elif variant == "alchemy":
+            g.set_alchemy(s.ss_alchemy, 0.5, 0.5)
+            g.set_lambda(0.0, 0.3, 0.0, 0.6)
+        g.set_pair_tuning(*cfg)
+        g.update_lists()
+        dev = torch.device("cuda", 0)
+        x, gr, mo = (torch.from_numpy(np.concatenate(a)).to(dev) for a in (
+            (g.xp0, g.yp0, g.zp0), (g.xpg, g.ypg, g.zpg), (g.xpcm, g.ypcm, g.zpcm)))
+        for energies in (True, False):
+            for sh in (b"m", b"l", b"h"):
+                f = torch.zeros(3 * s.ntap, dtype=torch.float64, device=dev)
+                e = torch.zeros(8, dtype=torch.float64, device=dev)
+                torch.cuda.synchronize()
+                rc = g.lib.orac_gpu_mts_forces_dev(g.ctx, sh, x.data_ptr(), gr.data_ptr(), mo.data_ptr(),
+                                                   f.data_ptr(), e.data_ptr() if energies else None, None)
+                assert rc == 0
+                torch.cuda.synchronize()
+                got.setdefault(sh, []).append(f.cpu().numpy())
+        g.close()
+    for sh, fs in got.items():
+        assert np.abs(fs[0]).max() > 0
+        for f in fs[1:]:
+            assert np.array_equal(f, fs[0]), sh
