@@ -274,7 +274,7 @@ int orac_gpu_destroy(orac_gpu_ctx* ctx) {
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
   md_destroy(ctx);
   void* ptrs[] = {ctx->d_gmeta, ctx->d_gpair, ctx->d_atype, ctx->d_apm, ctx->d_aq, ctx->d_aqd, ctx->d_amol, ctx->d_agrp,
-                  ctx->d_gmol, ctx->d_amassinf, ctx->d_lj, ctx->d_ljd, ctx->d_exoff, ctx->d_exj, ctx->d_xyz, ctx->d_grp,
+                  ctx->d_gmol, ctx->d_amassinf, ctx->d_lj, ctx->d_ljd, ctx->d_exoff, ctx->d_exj, ctx->d_exrange, ctx->d_xyz, ctx->d_grp,
                   ctx->d_mol, ctx->d_gpos, ctx->d_aoff, ctx->d_ffix, ctx->d_acc, ctx->d_fout, ctx->d_red,
                   ctx->d_scan_tmp, ctx->d_total, ctx->d_flag, ctx->d_cell_of, ctx->d_cell_cnt, ctx->d_cell_start,
                   ctx->d_cell_grp, ctx->d_stencil, ctx->pme.tw1, ctx->pme.tw2, ctx->pme.tw3, ctx->pme.bsp1,
@@ -434,6 +434,16 @@ int orac_gpu_set_topology(orac_gpu_ctx* ctx, int ntap, int ngrp, int nprot, cons
   UP(ctx->d_lj, lj);
   UP(ctx->d_ljd, ljd);
   UP(ctx->d_exoff, exoff);
+  {
+    std::vector<int2> ex(G, make_int2(N, -1));
+    for (int a = 0; a < N; a++)
+      for (int e = exoff[a]; e < exoff[a + 1]; e++) {
+        int2& r = ex[agrp[a]];
+        r.x = exj[e] < r.x ? exj[e] : r.x;
+        r.y = exj[e] > r.y ? exj[e] : r.y;
+      }
+    UP(ctx->d_exrange, ex);
+  }
   if (exj.empty()) exj.push_back(0);
   UP(ctx->d_exj, exj);
   std::vector<double> qd(chrge, chrge + N);

@@ -81,13 +81,12 @@ struct AlchDyn {
   double f[2][9], fq[2][9], f0[2][9], fq0[2][9], df[2][9], dfq[2][9];
 };
 
-// A group-pair list in CSR form with fixed row capacities: row i occupies
-// [off[i], off[i+1]) and holds cnt[i] entries.  Nested shell lists reuse the
-// rows of their parent list.
+// A group-pair list: row i holds cnt[i] entries from off[i].  Nested shell
+// lists reuse the rows of their parent list.
 struct GList {
-  int* off = nullptr;   // [ngrp+1]
+  int* off = nullptr;   // [ngrp] row starts, in any order
   int* cnt = nullptr;   // [ngrp]
-  int* j = nullptr;     // [cap] partner group, 0-based, > row group
+  int* j = nullptr;     // [cap] partner group, 0-based; a pair is in one of the two rows
   unsigned long long* mask = nullptr;  // [cap] skipped atom pairs, bit a*8+b
   int64_t cap = 0;
   int64_t npairs = 0;   // host copy, updated when read back
@@ -345,6 +344,7 @@ struct orac_gpu_ctx {
   double2* d_ljd = nullptr;
   int* d_exoff = nullptr;  // [N+1]
   int* d_exj = nullptr;    // 0-based partners j > i
+  int2* d_exrange = nullptr;  // [G] lowest and highest partner of a group's atoms
 
   // box and parameters
   double co[9] = {0}, oc[9] = {0}, volume = 0;

@@ -4,16 +4,18 @@
 //
 // ORAC bins group centres into ncx*ncy*ncz cells and, for every group n,
 // scans a precomputed stencil of cells keeping partners l > n whose
-// minimum-image centre distance is below rcut.  Here:
+// minimum-image centre distance is below rcut.  Here, where a pair is kept
+// once too, in one of the two groups' rows (keeps):
 //   k_cell_assign   cell of every group (ORAC's floor/wrap formula, FP64)
 //   k_scan          exclusive prefix sum (one block; lists are rebuilt every
 //                   few steps, so one block is enough)
 //   k_cell_fill     counting-sort placement, then k_cell_order sorts every
 //                   cell by group index so results do not depend on atomics
-//   k_pairs<FILL>   one warp per group, lanes over stencil cells; a count
-//                   pass sizes the CSR rows, the fill pass writes them in
-//                   stencil order and computes the exclusion masks of pairs
-//                   that belong to one molecule.
+//   k_pairs         one warp per group, lanes over stencil cells: the row's
+//                   partners are gathered in shared memory, its place in the
+//                   list is taken with one atomic, and the entries are written
+//                   with the exclusion masks of pairs that belong to one
+//                   molecule.
 // The stencil itself is built on the host with ORAC's dist_ijk criterion.
 #include <algorithm>
 #include <cmath>
@@ -120,7 +122,7 @@ struct ListArgs {
   const int* cell_grp;
   // outputs
   int* cnt;
-  const int* off;
+  int* off;
   int* j;
   unsigned long long* mask;
   // topology for masks
@@ -129,13 +131,33 @@ struct ListArgs {
   const int* exoff;
   const int* exj;
   const unsigned char* massinf;
+  const int2* exrange;  // [G] lowest and highest excluded partner of a group's atoms
   int allpairs;
-  int64_t cap;  // fill pass: entries available (negative: unchecked)
-  int* flag;    // fill pass: bit 1 set on overflow
+  int64_t cap;                // entries available
+  unsigned long long* total;  // entries of the rows so far (zeroed before)
+  int* flag;                  // bit 1 set where a row finds no room (null: not)
 };
 
+// Which of two groups keeps their pair in its row.  ORAC: the lower index.
+// Here: the one that has the other within half of the index circle ahead of
+// it, which is the lower index except across the circle's seam.  By plain
+// index the rows of a box's first groups hold the neighbours through the
+// periodic faces and those of its last ones none, and a pair kernel, with a
+// warp or half a warp a row, waits for the longest rows (3,000 waters, M list:
+// 0 to 35 entries, mean 12).  The rule depends on indices alone, so a list
+// built again gives every pair the same two roles and bitwise the same forces;
+// by turns of the parity the rows balance too, but hold both sides of a
+// group's surroundings, and the kernels of the longer lists read half as much
+// again (L shell 17.9 against 15.1 us).
+__device__ __forceinline__ bool keeps(int i, int l, int G) {
+  int d = l - i;
+  if (d < 0) d += G;
+  return d != 0 && (2 * d < G || (2 * d == G && i < l));
+}
+
 __device__ __forceinline__ bool pair_in(const ListArgs& A, double xi, double yi,
-                                        double zi, int l) {
+                                        double zi, int i, int l) {
+  if (!keeps(i, l, A.G)) return false;
   double dx = xi - A.grp[l], dy = yi - A.grp[A.G + l], dz = zi - A.grp[2 * A.G + l];
   dx -= 2.0 * round(0.5 * dx);  // pbc.h: anint(0.5 x)
   dy -= 2.0 * round(0.5 * dy);
@@ -151,8 +173,19 @@ __device__ __forceinline__ bool pair_in(const ListArgs& A, double xi, double yi,
 // are both >= massinfty (src/force.f:374-388, 486-489).
 __device__ unsigned long long pair_mask(const ListArgs& A, int i, int l) {
   if (A.gmol[i] != A.gmol[l]) return 0ull;
+  // mapnl lists each exclusion at the atom of lower index, and the fixed-mass
+  // rule is that group's: evaluated from there, and turned for the higher one
+  const bool turn = l < i;
+  if (turn) {
+    const int k = i;
+    i = l;
+    l = k;
+  }
   const int2 mi = A.gmeta[i], ml = A.gmeta[l];
   const int i0 = mi.x, ni = mi.y & 0xff, l0 = ml.x, nl = ml.y & 0xff;
+  // most groups of a large molecule lie beyond its excluded partners
+  const int2 ex = A.exrange[i];
+  if (l0 > ex.y || l0 + nl - 1 < ex.x) return 0ull;
   unsigned long long m = 0ull;
   for (int a = 0; a < ni; a++) {
     bool any = false;
@@ -167,81 +200,112 @@ __device__ unsigned long long pair_mask(const ListArgs& A, int i, int l) {
       for (int b = 0; b < nl; b++)
         if (A.massinf[l0 + b]) m |= 1ull << (a * 8 + b);
   }
+  if (turn && m) {
+    unsigned long long r = 0ull;
+    for (int k = 0; k < 64; k++) r |= ((m >> k) & 1ull) << ((k & 7) * 8 + (k >> 3));
+    m = r;
+  }
   return m;
 }
 
-// One warp per group i.  Count pass: cnt[i].  Fill pass: entries in stencil
-// order (lanes take 32 consecutive stencil cells, a warp scan orders their
-// hits), within a cell by group index.
-template <bool FILL>
+// One warp per group i, lanes over 32 stencil cells at a time (a cell holds
+// about one group): hits go to the row's buffer in shared memory by ballots,
+// in the order of stencil chunk, place in the cell and stencil cell.  The row
+// then takes its place in the list with one atomic on the list's length and
+// writes entries and masks; rows lie in any order, which nothing depends on.
+// A row without room is left empty and sets the flag; the length counts it all
+// the same, so a build into too small a list yields the size it needs.  A row
+// longer than the buffer is gathered a second time, straight into the list.
+// Bound by the latency of the chain stencil -> cell -> group -> centre: the
+// next cells are read ahead.  One pass where there were a count pass, a scan
+// and a fill pass that did the count's work again (3,000 waters: 31 + 5 + 45 us;
+// 14,900 atoms, whose masks were most of the fill: 48 + 6 + 114 us).
+constexpr int ROW_BUF = 512;
+
 __global__ void __launch_bounds__(128) k_pairs(const ListArgs A) {
   pdl_enter();
-  const int lane = threadIdx.x & 31;
-  const int i = blockIdx.x * 4 + (threadIdx.x >> 5);
+  constexpr unsigned FULL = 0xffffffffu;
+  __shared__ int s_hit[4][ROW_BUF];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = blockIdx.x * 4 + warp;
   if (i >= A.G) return;
-  if (FILL && A.cap >= 0 && (int64_t)A.off[A.G] > A.cap) {  // ORAC: xerror on nnlpp overflow
-    if (i == 0 && lane == 0) atomicOr(A.flag, 2);
-    return;
-  }
   const double xi = A.grp[i], yi = A.grp[A.G + i], zi = A.grp[2 * A.G + i];
-  int total = 0;
-  const int base = FILL ? A.off[i] : 0;
-  if (A.allpairs) {
-    for (int l0 = i + 1; l0 < A.G; l0 += 32) {
-      const int l = l0 + lane;
-      const bool hit = l < A.G && pair_in(A, xi, yi, zi, l);
-      const unsigned bal = __ballot_sync(0xffffffffu, hit);
-      if (FILL && hit) {
-        const int pos = base + total + __popc(bal & ((1u << lane) - 1u));
-        A.j[pos] = l;
-        A.mask[pos] = pair_mask(A, i, l);
+  const unsigned below = (1u << lane) - 1u;
+  int* hits = s_hit[warp];
+  const int c = A.allpairs ? 0 : A.cell_of[i];
+  const int ci = c / (A.ncy * A.ncz), cj = (c / A.ncz) % A.ncy, ck = c % A.ncz;
+  // the groups [cb, ce) of stencil cell s
+  auto cell = [&](int s, int* cb, int* ce) {
+    *cb = *ce = 0;
+    if (s >= A.nsten) return;
+    int nx = ci + A.stencil[3 * s], ny = cj + A.stencil[3 * s + 1], nz = ck + A.stencil[3 * s + 2];
+    // (a stencil offset is less than one box, src/lc_index.f:52-91)
+    nx += nx < 0 ? A.ncx : (nx >= A.ncx ? -A.ncx : 0);
+    ny += ny < 0 ? A.ncy : (ny >= A.ncy ? -A.ncy : 0);
+    nz += nz < 0 ? A.ncz : (nz >= A.ncz ? -A.ncz : 0);
+    const int cc = nz + A.ncz * (ny + A.ncy * nx);
+    *cb = A.cell_start[cc];
+    *ce = A.cell_start[cc + 1];
+  };
+  // runs put(l, place in the row) for the row's partners; returns their number
+  auto gather = [&](auto&& put) {
+    int total = 0;
+    if (A.allpairs) {
+      for (int l0 = 0; l0 < A.G; l0 += 32) {
+        const int l = l0 + lane;
+        const bool hit = l < A.G && pair_in(A, xi, yi, zi, i, l);
+        const unsigned bal = __ballot_sync(FULL, hit);
+        if (hit) put(l, total + __popc(bal & below));
+        total += __popc(bal);
       }
-      total += __popc(bal);
+      return total;
+    }
+    int cb, ce, nb, ne;
+    cell(lane, &nb, &ne);
+    int lnext = nb < ne ? A.cell_grp[nb] : -1;
+    for (int s0 = 0; s0 < A.nsten; s0 += 32) {
+      cb = nb;
+      ce = ne;
+      int l = lnext;
+      cell(s0 + 32 + lane, &nb, &ne);
+      lnext = nb < ne ? A.cell_grp[nb] : -1;
+      for (int p = cb; __any_sync(FULL, p < ce); p++) {
+        const int now = l;
+        l = p + 1 < ce ? A.cell_grp[p + 1] : -1;
+        const bool hit = p < ce && pair_in(A, xi, yi, zi, i, now);
+        const unsigned bal = __ballot_sync(FULL, hit);
+        if (hit) put(now, total + __popc(bal & below));
+        total += __popc(bal);
+      }
+    }
+    return total;
+  };
+  const int total = gather([&](int l, int k) {
+    if (k < ROW_BUF) hits[k] = l;
+  });
+  unsigned long long base = 0;
+  if (lane == 0) base = atomicAdd(A.total, (unsigned long long)total);
+  base = __shfl_sync(FULL, base, 0);
+  const bool fits = (int64_t)(base + total) <= A.cap;
+  if (lane == 0) {
+    A.off[i] = fits ? (int)base : 0;
+    A.cnt[i] = fits ? total : 0;
+    if (!fits && A.flag) atomicOr(A.flag, 2);  // ORAC: xerror on nnlpp overflow
+  }
+  if (!fits) return;
+  if (total <= ROW_BUF) {
+    __syncwarp();
+    for (int k = lane; k < total; k += 32) {
+      const int l = hits[k];
+      A.j[base + k] = l;
+      A.mask[base + k] = pair_mask(A, i, l);
     }
   } else {
-    const int c = A.cell_of[i];
-    const int ci = c / (A.ncy * A.ncz), cj = (c / A.ncz) % A.ncy, ck = c % A.ncz;
-    for (int s0 = 0; s0 < A.nsten; s0 += 32) {
-      const int s = s0 + lane;
-      int cb = 0, ce = 0;
-      if (s < A.nsten) {
-        int nx = (ci + A.stencil[3 * s]) % A.ncx;
-        if (nx < 0) nx += A.ncx;
-        int ny = (cj + A.stencil[3 * s + 1]) % A.ncy;
-        if (ny < 0) ny += A.ncy;
-        int nz = (ck + A.stencil[3 * s + 2]) % A.ncz;
-        if (nz < 0) nz += A.ncz;
-        const int cc = nz + A.ncz * (ny + A.ncy * nx);
-        cb = A.cell_start[cc];
-        ce = A.cell_start[cc + 1];
-      }
-      int mine = 0;
-      for (int p = cb; p < ce; p++) {
-        const int l = A.cell_grp[p];
-        if (l > i && pair_in(A, xi, yi, zi, l)) mine++;
-      }
-      // exclusive warp scan of the per-lane hit counts
-      int incl = mine;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-      }
-      if (FILL && mine) {
-        int pos = base + total + incl - mine;
-        for (int p = cb; p < ce; p++) {
-          const int l = A.cell_grp[p];
-          if (l > i && pair_in(A, xi, yi, zi, l)) {
-            A.j[pos] = l;
-            A.mask[pos] = pair_mask(A, i, l);
-            pos++;
-          }
-        }
-      }
-      total += __shfl_sync(0xffffffffu, incl, 31);
-    }
+    gather([&](int l, int k) {
+      A.j[base + k] = l;
+      A.mask[base + k] = pair_mask(A, i, l);
+    });
   }
-  if (!FILL && lane == 0) A.cnt[i] = total;
 }
 
 // dist_ijk (src/dist_ijk.f:3-141): squared minimum distance between cell
@@ -355,23 +419,32 @@ ListArgs base_args(orac_gpu_ctx* ctx, double rcut, GList* out) {
   A.exoff = ctx->d_exoff;
   A.exj = ctx->d_exj;
   A.massinf = ctx->d_amassinf;
-  A.cap = -1;
-  A.flag = ctx->d_flag;
+  A.exrange = ctx->d_exrange;
+  A.cap = out->cap;
+  A.total = reinterpret_cast<unsigned long long*>(ctx->d_total);
+  A.j = out->j;
+  A.mask = out->mask;
+  A.flag = nullptr;
   return A;
 }
 
-// count -> scan -> (grow) -> fill
-int pairs_count_fill(orac_gpu_ctx* ctx, ListArgs A, GList* out) {
-  const int nb = (ctx->G + 3) / 4;
-  orac_launch(k_pairs<false>, nb, 128, 0, ctx->stream, A);
+int pairs_launch(orac_gpu_ctx* ctx, const ListArgs& A) {
+  CK(cudaMemsetAsync(A.total, 0, sizeof(unsigned long long), ctx->stream));
+  orac_launch(k_pairs, (ctx->G + 3) / 4, 128, 0, ctx->stream, A);
   CKL();
-  orac_launch(k_scan, 1, 1024, 0, ctx->stream, ctx->G, out->cnt, out->off, ctx->d_total);
-  CKL();
-  int64_t total = 0;
-  CK(cudaMemcpyAsync(&total, ctx->d_total, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
-  if (total >= (int64_t)1 << 31) return ctx_fail(ctx, ORAC_ERR_CAPACITY, "neighbour list of %lld pairs", (long long)total);
-  if (total > out->cap) {
+  return ORAC_OK;
+}
+
+// build, and once more where the list had to grow to the length found
+int pairs_build(orac_gpu_ctx* ctx, ListArgs A, GList* out) {
+  for (;;) {
+    if (int rc = pairs_launch(ctx, A)) return rc;
+    int64_t total = 0;
+    CK(cudaMemcpyAsync(&total, ctx->d_total, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    if (total >= (int64_t)1 << 31) return ctx_fail(ctx, ORAC_ERR_CAPACITY, "neighbour list of %lld pairs", (long long)total);
+    out->npairs = total;
+    if (total <= out->cap) break;
     const int64_t cap = total + total / 4 + 1024;
     if (dev_alloc(ctx, &out->j, cap)) return ORAC_ERR_CUDA;
     if (dev_alloc(ctx, &out->mask, cap)) return ORAC_ERR_CUDA;
@@ -384,12 +457,10 @@ int pairs_count_fill(orac_gpu_ctx* ctx, ListArgs A, GList* out) {
       L.cap = cap;
       L.valid = false;
     }
+    A.cap = cap;
+    A.j = out->j;
+    A.mask = out->mask;
   }
-  A.j = out->j;
-  A.mask = out->mask;
-  orac_launch(k_pairs<true>, nb, 128, 0, ctx->stream, A);
-  CKL();
-  out->npairs = total;
   out->valid = true;
   ctx->lists[1].valid = false;
   ctx->lists[2].valid = false;
@@ -421,13 +492,13 @@ int list_build_cells(orac_gpu_ctx* ctx, double rcut, GList* out) {
   CKL();
   ListArgs A = base_args(ctx, rcut, out);
   A.allpairs = 0;
-  return pairs_count_fill(ctx, A, out);
+  return pairs_build(ctx, A, out);
 }
 
 int list_build_allpairs(orac_gpu_ctx* ctx, double rcut, GList* out) {
   ListArgs A = base_args(ctx, rcut, out);
   A.allpairs = 1;
-  return pairs_count_fill(ctx, A, out);
+  return pairs_build(ctx, A, out);
 }
 
 int list_prepare_stencil(orac_gpu_ctx* ctx, double rcut) {
@@ -460,17 +531,8 @@ int list_build_cells_async(orac_gpu_ctx* ctx, double rcut, GList* out, int* d_fl
   CKL();
   ListArgs A = base_args(ctx, rcut, out);
   A.allpairs = 0;
-  A.cap = out->cap;
   A.flag = d_flag;
-  const int nb = (G + 3) / 4;
-  orac_launch(k_pairs<false>, nb, 128, 0, ctx->stream, A);
-  CKL();
-  orac_launch(k_scan, 1, 1024, 0, ctx->stream, G, out->cnt, out->off, ctx->d_total);
-  CKL();
-  A.j = out->j;
-  A.mask = out->mask;
-  orac_launch(k_pairs<true>, nb, 128, 0, ctx->stream, A);
-  CKL();
+  if (int rc = pairs_launch(ctx, A)) return rc;
   out->valid = true;
   return ORAC_OK;
 }
