@@ -577,7 +577,8 @@ int pme_run(orac_gpu_ctx* ctx, int natom, const double* d_cart /*3N*/,
             unsigned long long* d_ffix = nullptr /*3N fixed point instead of d_f*/,
             const double* d_dq = nullptr, double* d_edq = nullptr /*sum phi_i dq_i, accumulated*/,
             float2* d_save = nullptr /*keep the transformed grid (h1 n2 n3)*/,
-            const float2* d_cross = nullptr /*energy difference against a kept grid, no forces*/);
+            const float2* d_cross = nullptr /*energy difference against a kept grid, no forces*/,
+            bool sums = true /*the energy and virial sums into d_eout*/);
 // k_small.cu: kind 0 fnb14, 1 fnbgrp, 2 ferrf; d_e[4]
 int small_launch(orac_gpu_ctx* ctx, int kind, const double* d_xyz,
                  const int* d_pairs, const int* d_ptype, int npairs,

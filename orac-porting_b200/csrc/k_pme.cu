@@ -95,7 +95,7 @@ __device__ __forceinline__ float2 twid(const float2* tw, int k, int sign) {
 // the twiddles W_n^(k r tsc) with k = j mod Ns, and writes the R-point DFT
 // to b[l][(j/Ns) Ns R + k + q Ns].
 template <int R>
-__device__ __forceinline__ void fft_pass(const float2* __restrict__ in, float2* __restrict__ out, int nl, int n,
+__device__ __forceinline__ void fft_pass(const float2* __restrict__ in, float2* __restrict__ out, int nl, int stride,
                                          const FftPlan& P, int s, const float2* tw, int sign) {
   const int nb = P.nb[s], Ns = P.ns[s], tsc = P.tsc[s];
   const unsigned mnb = P.mnb[s], mns = P.mns[s];
@@ -107,7 +107,7 @@ __device__ __forceinline__ void fft_pass(const float2* __restrict__ in, float2* 
     const int l = qdiv(t, mnb), j = t - l * nb;
     const int jq = qdiv(j, mns), k = j - jq * Ns;
     const int tstep = k * tsc;
-    const float2* src = in + l * n + j;
+    const float2* src = in + l * stride + j;
     float2 v[R];
 #pragma unroll
     for (int r = 0; r < R; r++) {
@@ -115,7 +115,7 @@ __device__ __forceinline__ void fft_pass(const float2* __restrict__ in, float2* 
       if (r && tstep) x = cmul(x, twid(tw, tstep * r, sign));
       v[r] = x;
     }
-    float2* dst = out + l * n + jq * Ns * R + k;
+    float2* dst = out + l * stride + jq * Ns * R + k;
     if (R == 2) {
       dst[0] = cadd(v[0], v[1]);
       dst[Ns] = csub(v[0], v[1]);
@@ -140,17 +140,16 @@ __device__ __forceinline__ void fft_pass(const float2* __restrict__ in, float2* 
   }
 }
 
-// Stockham passes over `nl` lines of length n stored line-major in a; the
-// result ends in the returned buffer (a or b).
-__device__ float2* fft_smem(float2* a, float2* b, int nl, const FftPlan& P, const float2* tw, int sign) {
-  const int n = P.n;
+// Stockham passes over `nl` lines of P.n values, `stride` apart, stored
+// line-major in a; the result ends in the returned buffer (a or b).
+__device__ float2* fft_smem(float2* a, float2* b, int nl, int stride, const FftPlan& P, const float2* tw, int sign) {
   for (int s = 0; s < P.nst; s++) {
     switch (P.rad[s]) {
-      case 4: fft_pass<4>(a, b, nl, n, P, s, tw, sign); break;
-      case 2: fft_pass<2>(a, b, nl, n, P, s, tw, sign); break;
-      case 3: fft_pass<3>(a, b, nl, n, P, s, tw, sign); break;
-      case 5: fft_pass<5>(a, b, nl, n, P, s, tw, sign); break;
-      default: fft_pass<7>(a, b, nl, n, P, s, tw, sign); break;
+      case 4: fft_pass<4>(a, b, nl, stride, P, s, tw, sign); break;
+      case 2: fft_pass<2>(a, b, nl, stride, P, s, tw, sign); break;
+      case 3: fft_pass<3>(a, b, nl, stride, P, s, tw, sign); break;
+      case 5: fft_pass<5>(a, b, nl, stride, P, s, tw, sign); break;
+      default: fft_pass<7>(a, b, nl, stride, P, s, tw, sign); break;
     }
     __syncthreads();
     float2* t = a;
@@ -205,21 +204,30 @@ struct GridArgs {
   // |S|^2 - |S - T|^2 = 2 Re(S conj T) - |T|^2 of this grid T and stops
   float2* save;
   const float2* cross;
+  int early;  // pdl_release
+  // the z pass sums the energy and virial into eout (0: potential only)
+  int sums;
+  // the plane passes: the y axis' twiddles and plan beside tw and P (the x
+  // axis')
+  const float2* twy;
+  FftPlan PY;
 };
 
 enum { XF = 0, YF = 1, ZC = 2, YI = 3, XI = 4 };
 
 template <int MODE>
 __global__ void __launch_bounds__(FFT_THREADS) k_fft(const GridArgs A) {
-  pdl_enter();
   extern __shared__ float2 sm[];
   const int n = A.P.n;
   const int B = A.B;
   float2* a = sm;
   float2* b = sm + B * n;
-  // the line's twiddles, staged after the two line buffers
+  // the line's twiddles, staged after the two line buffers (no kernel writes
+  // them: before the wait)
   float2* tws = sm + 2 * B * n;
   for (int e = threadIdx.x; e < n; e += blockDim.x) tws[e] = A.tw[e];
+  pdl_enter();
+  pdl_release(A.early);
   // line geometry
   int nlines, i0 = 0, j0 = 0, k0 = 0, nl;
   if (MODE == XF || MODE == XI) {
@@ -274,7 +282,7 @@ __global__ void __launch_bounds__(FFT_THREADS) k_fft(const GridArgs A) {
   }
   __syncthreads();
   const int sign = (MODE == XF || MODE == YF) ? -1 : +1;
-  float2* res = fft_smem(a, b, nl, A.P, tws, MODE == ZC ? -1 : sign);
+  float2* res = fft_smem(a, b, nl, n, A.P, tws, MODE == ZC ? -1 : sign);
   if (MODE == ZC) {
     // influence function, src/scalar_sum.f:40-121 (element (1,1,1) untouched)
     double acc[7] = {0, 0, 0, 0, 0, 0, 0};
@@ -304,6 +312,10 @@ __global__ void __launch_bounds__(FFT_THREADS) k_fft(const GridArgs A) {
         const float fm = (float)msq;
         const float denom = A.pivol * A.bsp1[k1 - 1] * A.bsp2[k2 - 1] * A.bsp3[k3 - 1] * fm;
         eterm = expf(-A.fac * fm) / denom;
+        if (!A.sums) {
+          res[e] = make_float2(q.x * eterm, q.y * eterm);
+          continue;
+        }
         const double vterm = 2.0 * ((double)A.fac * msq + 1.0) / msq;
         double q2 = (double)q.x * q.x + (double)q.y * q.y;
         if (A.cross) {
@@ -340,10 +352,10 @@ __global__ void __launch_bounds__(FFT_THREADS) k_fft(const GridArgs A) {
       res[e] = make_float2(q.x * eterm, q.y * eterm);
     }
     __syncthreads();
-    block_reduce_add<7>(acc, A.eout);
+    if (A.sums) block_reduce_add<7>(acc, A.eout);
     if (A.cross) return;  // the energy difference alone
     float2* other = (res == a) ? b : a;
-    res = fft_smem(res, other, nl, A.P, tws, +1);
+    res = fft_smem(res, other, nl, n, A.P, tws, +1);
   }
   // ---- store
   if (MODE == XF) {
@@ -368,6 +380,110 @@ __global__ void __launch_bounds__(FFT_THREADS) k_fft(const GridArgs A) {
   }
 }
 
+// The x and y passes of one z plane in one block, the plane in shared memory:
+// forward (INV 0) from the charge grid to the half spectrum, and back (INV 1)
+// to the real grid.  Two real x lines ride in one complex line (rows 2p and
+// 2p + 1 as real and imaginary part), so the x pass transforms half as many.
+// The lines' strides are odd: the transposition between the x and y lines
+// reads and writes without bank conflicts.  In place of two kernels a way
+// (k_fft<XF>, <YF> and <YI>, <XI>), whose passes over these grids (48^3 to
+// 96^3, a few MB in L2) were latency and launches: an SPME evaluation of 9,000
+// atoms on 48^3 took 7 kernels and two clears, now 5 and one.
+template <int INV>
+__global__ void __launch_bounds__(1024) k_plane(const GridArgs A) {
+  extern __shared__ float2 sm[];
+  const int n1 = A.n1, n2 = A.n2, h1 = A.h1, hx = (n2 + 1) / 2;
+  const int S1 = n1 | 1, S2 = n2 | 1;
+  const int cap = max(hx * S1, h1 * S2);
+  float2* a = sm;
+  float2* b = sm + cap;
+  float2* twx = sm + 2 * cap;
+  float2* twy = twx + n1;
+  for (int e = threadIdx.x; e < n1; e += blockDim.x) twx[e] = A.tw[e];
+  for (int e = threadIdx.x; e < n2; e += blockDim.x) twy[e] = A.twy[e];
+  pdl_enter();
+  pdl_release(A.early);
+  const int k0 = blockIdx.x;
+  const unsigned mh1 = h1 == 1 ? 0u : (unsigned)((1ull << 32) / (unsigned)h1 + 1ull);
+  const unsigned mhx = hx == 1 ? 0u : (unsigned)((1ull << 32) / (unsigned)hx + 1ull);
+  if (INV == 0) {
+    const unsigned long long* src = A.qfix + (size_t)k0 * n2 * n1;
+#pragma unroll 4
+    for (int e = threadIdx.x; e < hx * n1; e += blockDim.x) {
+      const int p = qdiv(e, A.P.mn), i = e - p * n1;
+      const long long q0 = (long long)src[2 * p * n1 + i];
+      const long long q1 = 2 * p + 1 < n2 ? (long long)src[(2 * p + 1) * n1 + i] : 0ll;
+      a[p * S1 + i] = make_float2((float)((double)q0 * (1.0 / ORAC_QSCALE)), (float)((double)q1 * (1.0 / ORAC_QSCALE)));
+    }
+    __syncthreads();
+    float2* r = fft_smem(a, b, hx, S1, A.P, twx, -1);
+    float2* y = r == a ? b : a;
+    // the two lines' half spectra, turned into y lines
+    for (int e = threadIdx.x; e < hx * h1; e += blockDim.x) {
+      const int i = qdiv(e, mhx), p = e - i * hx;
+      const float2 z = r[p * S1 + i], w = r[p * S1 + (i ? n1 - i : 0)];
+      y[i * S2 + 2 * p] = make_float2(0.5f * (z.x + w.x), 0.5f * (z.y - w.y));
+      if (2 * p + 1 < n2) y[i * S2 + 2 * p + 1] = make_float2(0.5f * (z.y + w.y), 0.5f * (w.x - z.x));
+    }
+    __syncthreads();
+    r = fft_smem(y, y == a ? b : a, h1, S2, A.PY, twy, -1);
+    float2* dst = A.cg + (size_t)k0 * n2 * h1;
+#pragma unroll 4
+    for (int e = threadIdx.x; e < n2 * h1; e += blockDim.x) {
+      const int j = qdiv(e, mh1), i = e - j * h1;
+      dst[e] = r[i * S2 + j];
+    }
+  } else {
+    const float2* src = A.cg + (size_t)k0 * n2 * h1;
+#pragma unroll 4
+    for (int e = threadIdx.x; e < n2 * h1; e += blockDim.x) {
+      const int j = qdiv(e, mh1), i = e - j * h1;
+      a[i * S2 + j] = src[e];
+    }
+    __syncthreads();
+    float2* r = fft_smem(a, b, h1, S2, A.PY, twy, +1);
+    float2* x = r == a ? b : a;
+    // lines 2p + i (2p + 1), with the Hermitian half filled in; the real parts
+    // that c2r keeps take no part of the imaginary parts of the terms 0 and
+    // n1/2, which are rounding
+    for (int e = threadIdx.x; e < hx * n1; e += blockDim.x) {
+      const int i = qdiv(e, mhx), p = e - i * hx;
+      const bool up = i >= h1;
+      const int ii = up ? n1 - i : i;
+      float2 u = r[ii * S2 + 2 * p];
+      float2 w = 2 * p + 1 < n2 ? r[ii * S2 + 2 * p + 1] : make_float2(0.f, 0.f);
+      if (ii == 0 || 2 * ii == n1) u.y = w.y = 0.f;
+      x[p * S1 + i] = up ? make_float2(u.x + w.y, w.x - u.y) : make_float2(u.x - w.y, u.y + w.x);
+    }
+    __syncthreads();
+    r = fft_smem(x, x == a ? b : a, hx, S1, A.P, twx, +1);
+    float* dst = A.rg + (size_t)k0 * n2 * n1;
+    for (int e = threadIdx.x; e < hx * n1; e += blockDim.x) {
+      const int p = qdiv(e, A.P.mn), i = e - p * n1;
+      const float2 v = r[p * S1 + i];
+      dst[2 * p * n1 + i] = v.x;
+      if (2 * p + 1 < n2) dst[(2 * p + 1) * n1 + i] = v.y;
+    }
+  }
+}
+
+// shared memory of k_plane, and the largest that is used (two blocks of it
+// stay resident on an SM); larger planes take the separate x and y passes
+size_t plane_smem(int n1, int n2) {
+  const size_t hx = (n2 + 1) / 2, h1 = n1 / 2 + 1, s1 = n1 | 1, s2 = n2 | 1;
+  const size_t cap = hx * s1 > h1 * s2 ? hx * s1 : h1 * s2;
+  return (2 * cap + n1 + n2) * sizeof(float2);
+}
+constexpr size_t PLANE_SMEM_MAX = 112 * 1024;
+
+// threads of a plane's block: two for each radix-4 butterfly of the x pass (the
+// loads, the transposition and the stores take as many), up to 1,024
+int plane_threads(int n1, int n2) {
+  const int tot = ((n2 + 1) / 2) * n1 / 2;
+  const int th = (tot + 31) / 32 * 32;
+  return th < 64 ? 64 : (th > 1024 ? 1024 : th);
+}
+
 struct AtomArgs {
   int natom, order, n1, n2, n3;
   const double* xyz;  // [3N] Cartesian
@@ -388,6 +504,7 @@ struct AtomArgs {
   // reciprocal potential at atom i (dE/dq_i), into *edq (both null: off)
   const double* dq;
   double* edq;
+  int early;  // pdl_release
 };
 
 // fill_bspline restated in FP32 (src/pme_fftw3.f90:518-576).  P > 0: the
@@ -456,6 +573,7 @@ __device__ __forceinline__ int gidx(int k0, int n) {
 template <int P>
 __global__ void k_spread(const AtomArgs A) {
   pdl_enter();
+  pdl_release(A.early);
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int p = P > 0 ? P : A.order;
   if (t >= A.natom * p) return;
@@ -694,6 +812,10 @@ int pme_setup(orac_gpu_ctx* ctx, int n1, int n2, int n3, int order) {
   CK(cudaMemcpy(P.bsp1, b1.data(), sizeof(float) * n1, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(P.bsp2, b2.data(), sizeof(float) * n2, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(P.bsp3, b3.data(), sizeof(float) * n3, cudaMemcpyHostToDevice));
+  if (plane_smem(n1, n2) <= PLANE_SMEM_MAX) {  // (set here: not inside a capture)
+    CK(cudaFuncSetAttribute(k_plane<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PLANE_SMEM_MAX));
+    CK(cudaFuncSetAttribute(k_plane<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PLANE_SMEM_MAX));
+  }
   const size_t ng = (size_t)n1 * n2 * n3;
   if (dev_alloc(ctx, &P.qfix, ng) || dev_alloc(ctx, &P.rgrid, ng) || dev_alloc(ctx, &P.cgrid, (size_t)P.h1 * n2 * n3))
     return ORAC_ERR_CUDA;
@@ -703,12 +825,12 @@ int pme_setup(orac_gpu_ctx* ctx, int n1, int n2, int n3, int order) {
 int pme_run(orac_gpu_ctx* ctx, int natom, const double* d_cart, const double* d_q, const double* recip,
             double volume, double alpha, double* d_f, double* d_eout, const double* d_sxyz, const double* d_mol,
             unsigned long long* d_ffix, const double* d_dq, double* d_edq, float2* d_save,
-            const float2* d_cross) {
+            const float2* d_cross, bool sums) {
   PmePlan& P = ctx->pme;
   if (!P.qfix) return ctx_fail(ctx, ORAC_ERR_STATE, "PME not set up");
   const int n1 = P.n1, n2 = P.n2, n3 = P.n3, h1 = P.h1;
   CK(cudaMemsetAsync(P.qfix, 0, sizeof(unsigned long long) * (size_t)n1 * n2 * n3, ctx->stream));
-  CK(cudaMemsetAsync(d_eout, 0, sizeof(double) * 16, ctx->stream));
+  if (sums) CK(cudaMemsetAsync(d_eout, 0, sizeof(double) * 16, ctx->stream));
   AtomArgs A;
   memset(&A, 0, sizeof(A));
   A.natom = natom;
@@ -744,6 +866,7 @@ int pme_run(orac_gpu_ctx* ctx, int natom, const double* d_cart, const double* d_
   A.eout = d_eout;
   A.dq = d_edq ? d_dq : nullptr;
   A.edq = d_edq;
+  A.early = orac_early(ctx);
   const int nsp = natom * P.order;
   orac_launch(spread_kernel(P.order), (nsp + 255) / 256, 256, 0, ctx->stream, A);
   CKL();
@@ -775,9 +898,20 @@ int pme_run(orac_gpu_ctx* ctx, int natom, const double* d_cart, const double* d_
   G.eout = d_eout;
   G.save = d_save;
   G.cross = d_cross;
+  G.early = orac_early(ctx);
+  G.sums = sums ? 1 : 0;
   int nb;
   size_t sm;
-  {
+  const size_t psm = plane_smem(n1, n2);
+  const bool planes = psm <= PLANE_SMEM_MAX;
+  if (planes) {
+    make_plan(n1, &G.P);
+    make_plan(n2, &G.PY);
+    G.tw = P.tw1;
+    G.twy = P.tw2;
+    orac_launch(k_plane<0>, n3, plane_threads(n1, n2), psm, ctx->stream, G);
+    CKL();
+  } else {
     // x forward (r2c)
     make_plan(n1, &G.P);
     G.tw = P.tw1;
@@ -806,7 +940,12 @@ int pme_run(orac_gpu_ctx* ctx, int natom, const double* d_cart, const double* d_
   // the energy alone (the second charge set of a non-equilibrium step's
   // work): no potential back on the grid, no gather
   if (d_cross || (!d_f && !d_ffix && !d_edq && !(d_sxyz && d_mol))) return ORAC_OK;
-  {
+  if (planes) {
+    make_plan(n1, &G.P);
+    G.tw = P.tw1;
+    orac_launch(k_plane<1>, n3, plane_threads(n1, n2), psm, ctx->stream, G);
+    CKL();
+  } else {
     // y inverse
     make_plan(n2, &G.P);
     G.tw = P.tw2;
@@ -1080,6 +1219,7 @@ extern "C" int orac_gpu_pme_kspace_static(void* stream, int numatoms, const doub
   G.r33 = recip[8];
   const double pif = (double)3.14159265358979323846f;  // scalar_sum's single-precision pi
   const double rk = rkcut > 0.0 ? rkcut : 1e9;
+  G.sums = 1;
   G.fac = (float)(pif * pif / (ewald_coeff * ewald_coeff));
   G.pivol = (float)(pif * volume);
   G.rkcut2 = 0.25 * rk * rk / (pif * pif);

@@ -1990,7 +1990,7 @@ static int md_shell_recip(orac_gpu_ctx* ctx, MdState& S, char sh, int lvl, bool 
   // along a schedule the transformed grid of chrgec is kept for the work
   float2* keep = md_ne(ctx) ? ctx->pme.cgsave : nullptr;
   if (int rc = pme_run(ctx, ctx->N, S.x, ctx->pme_q(), recip, ctx->volume, ctx->alphal, nullptr, S.e + 24, nullptr,
-                       nullptr, f, dudl ? ctx->d_dq : nullptr, dudl ? S.e + E_DUDL + 3 : nullptr, keep))
+                       nullptr, f, dudl ? ctx->d_dq : nullptr, dudl ? S.e + E_DUDL + 3 : nullptr, keep, nullptr, energy))
     return rc;
   if (int rc = prof_end(ctx, slot)) return rc;
   if (!md_ne(ctx)) return md_ferrf(ctx, S, f, energy);
@@ -2402,7 +2402,15 @@ int orac_gpu_md_setup(orac_gpu_ctx* ctx, const double* x, const double* y, const
   MdState& S = *md_of(ctx);
   const int N = ctx->N, P = ctx->P, G = ctx->G;
   S.N = N;
-  CK(cudaStreamCreateWithFlags(&S.side, cudaStreamNonBlocking));
+  {
+    // the side stream's chain (SPME, a handful of small grids one after
+    // another) is the longest of a reciprocal level: its blocks go before
+    // those of the shells' pair kernels, which fill every SM otherwise and
+    // held it up (9,000 atoms: the last drift's SPME began 19 us late)
+    int lo = 0, hi = 0;
+    CK(cudaDeviceGetStreamPriorityRange(&lo, &hi));
+    CK(cudaStreamCreateWithPriority(&S.side, cudaStreamNonBlocking, hi));
+  }
   CK(cudaMallocHost((void**)&S.h_flag, sizeof(int)));
   CK(cudaEventCreateWithFlags(&S.ev_fork, cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&S.ev_join, cudaEventDisableTiming));

@@ -106,3 +106,27 @@ def test_forces_do_not_depend_on_energies_or_lanes(variant):
         assert np.abs(fs[0]).max() > 0
         for f in fs[1:]:
             assert np.array_equal(f, fs[0]), sh
+
+
+@pytest.mark.parametrize("nfft,order", [((8, 9, 10), 4), ((27, 35, 20), 5), ((30, 7, 25), 6), ((48, 49, 48), 4),
+                                        ((96, 96, 14), 8), ((160, 162, 9), 4), ((210, 8, 12), 7)])
+def test_plane_fft_grids(nfft, order):
+    """Odd axes, an odd number of x lines, planes at and beyond the shared
+    memory that the plane kernel uses."""
+    from orac_b200.engine import Engine
+
+    rng = np.random.default_rng(sum(nfft))
+    n = 300
+    box = np.array([14.0, 15.0, 13.0])
+    x = rng.uniform(-0.6, 0.6, (3, n)) * box[:, None]
+    q = rng.normal(0, 0.4, n)
+    q -= q.mean()
+    s = systems.two_waters()
+    g, o = Engine(s.copy()), oracle.Oracle(s.copy())
+    a = (x[0], x[1], x[2], q, np.diag(1.0 / box), float(box.prod()), 0.5)
+    Fg, eg, vg = g.do_pmesh_kspace(*a, order, nfft)
+    Fr, er, vr = o.do_pmesh_kspace(*a, order, nfft)[:3]
+    assert rel_rms(Fg, Fr) <= 1e-5
+    assert abs(eg - er) <= 1e-6 * abs(er)
+    assert np.linalg.norm(vg - np.asarray(vr).reshape(3, 3)) <= 1e-5 * np.linalg.norm(vr)
+    g.close()
