@@ -165,6 +165,7 @@ struct MolArgs {
   const unsigned long long* msum;
   const double* bmass;
   double tcm;
+  int early;  // release the next grid after the wait (pdl_release)
 };
 
 // a constraint cluster of a large molecule (the atoms joined by one
@@ -371,28 +372,38 @@ __device__ __forceinline__ bool shake_small(double x[SMA][3], const double xo[SM
 // (a heavy atom with its hydrogens).  The same Newton SHAKE and exact
 // RATTLE as shake_small / rattle_small with the topology known at compile
 // time: J_kl = 2 (im_0 + [k == l] im_{k+1}) d_k . r0_l.
+// (adjugate over determinant: one division, where elimination takes six in a
+// chain, which set the time of a thread with a three-hydrogen cluster)
 template <int NC>
 __device__ __forceinline__ bool solve_n(double A[NC][NC], double b[NC]) {
-#pragma unroll
-  for (int k = 0; k < NC; k++) {
-    if (A[k][k] == 0.0) return false;
-    const double inv = 1.0 / A[k][k];
-#pragma unroll
-    for (int i = k + 1; i < NC; i++) {
-      const double f = A[i][k] * inv;
-#pragma unroll
-      for (int j = k; j < NC; j++) A[i][j] -= f * A[k][j];
-      b[i] -= f * b[k];
-    }
+  if constexpr (NC == 1) {
+    if (A[0][0] == 0.0) return false;
+    b[0] = b[0] / A[0][0];
+    return true;
+  } else if constexpr (NC == 2) {
+    const double det = A[0][0] * A[1][1] - A[0][1] * A[1][0];
+    if (det == 0.0) return false;
+    const double id = 1.0 / det;
+    const double b0 = (A[1][1] * b[0] - A[0][1] * b[1]) * id;
+    b[1] = (A[0][0] * b[1] - A[1][0] * b[0]) * id;
+    b[0] = b0;
+    return true;
+  } else {
+    const double c00 = A[1][1] * A[2][2] - A[1][2] * A[2][1], c01 = A[1][2] * A[2][0] - A[1][0] * A[2][2],
+                 c02 = A[1][0] * A[2][1] - A[1][1] * A[2][0];
+    const double det = A[0][0] * c00 + A[0][1] * c01 + A[0][2] * c02;
+    if (det == 0.0) return false;
+    const double id = 1.0 / det;
+    const double b0 = (c00 * b[0] + (A[0][2] * A[2][1] - A[0][1] * A[2][2]) * b[1] +
+                       (A[0][1] * A[1][2] - A[0][2] * A[1][1]) * b[2]) * id;
+    const double b1 = (c01 * b[0] + (A[0][0] * A[2][2] - A[0][2] * A[2][0]) * b[1] +
+                       (A[0][2] * A[1][0] - A[0][0] * A[1][2]) * b[2]) * id;
+    b[2] = (c02 * b[0] + (A[0][1] * A[2][0] - A[0][0] * A[2][1]) * b[1] +
+            (A[0][0] * A[1][1] - A[0][1] * A[1][0]) * b[2]) * id;
+    b[0] = b0;
+    b[1] = b1;
+    return true;
   }
-#pragma unroll
-  for (int k = NC - 1; k >= 0; k--) {
-    double t = b[k];
-#pragma unroll
-    for (int j = k + 1; j < NC; j++) t -= A[k][j] * b[j];
-    b[k] = t / A[k][k];
-  }
-  return true;
 }
 
 template <int NC>
@@ -612,15 +623,66 @@ __device__ __forceinline__ void cross3(const double* a, const double* b, double*
   c[2] = a[0] * b[1] - a[1] * b[0];
 }
 
-__device__ bool settle3(double x[SMA][3], const double xo[SMA][3], double v[SMA][3], const double im[SMA],
-                        const double* L2, double idt) {
+// What SETTLE and the RATTLE after it take from a molecule's masses and lengths
+// alone: computed before the wait for the preceding grid.
+struct RigidIso {
+  bool ok;
+  double wA, wB, rc, ra, rb, ira, irc2;
+  double Mi[3][3];  // inverse of RATTLE's matrix cc_kl r_k . r_l at the constrained geometry
+};
+
+__device__ __forceinline__ void rigid_iso(const double im[SMA], const double* L2, RigidIso& K) {
   // mass fractions from the inverse masses: mA / (mA + 2 mB) = imB / (imB + 2 imA)
   const double iM = 1.0 / (im[1] + 2.0 * im[0]);
-  const double wA = im[1] * iM, wB = im[0] * iM;
-  const double rc = 0.5 * sqrt(L2[2]);
-  const double h2 = L2[0] - rc * rc;
-  if (!(h2 > 0.0)) return false;
-  const double h = sqrt(h2), ra = 2.0 * wB * h, rb = wA * h;  // apex and base from the centre of mass
+  K.wA = im[1] * iM;
+  K.wB = im[0] * iM;
+  K.rc = 0.5 * sqrt(L2[2]);
+  const double h2 = L2[0] - K.rc * K.rc;
+  K.ok = h2 > 0.0;
+  const double h = sqrt(h2 > 0.0 ? h2 : 1.0);  // apex and base from the centre of mass
+  K.ra = 2.0 * K.wB * h;
+  K.rb = K.wA * h;
+  K.ira = 1.0 / K.ra;
+  K.irc2 = 1.0 / (2.0 * K.rc);
+  // r0 = x0 - x1, r1 = x0 - x2, r2 = x1 - x2 = r1 - r0
+  const double half = 0.5 * L2[2];
+  const double g[3][3] = {{L2[0], L2[0] - half, -half}, {L2[0] - half, L2[0], half}, {-half, half, L2[2]}};
+  double cc[3][3];
+  coupling3(im, cc);
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    double M[3][3], e[3], col[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      e[k] = k == c ? 1.0 : 0.0;
+#pragma unroll
+      for (int l = 0; l < 3; l++) M[k][l] = cc[k][l] * g[k][l];
+    }
+    K.ok = solve3x3(M, e, col) && K.ok;
+#pragma unroll
+    for (int k = 0; k < 3; k++) K.Mi[k][c] = col[k];
+  }
+}
+
+// rattle3 of a molecule at its constrained geometry (SETTLE's result)
+__device__ __forceinline__ void rattle_iso(const double x[SMA][3], double v[SMA][3], const double im[SMA],
+                                           const RigidIso& K) {
+  double r[3][3], rhs[3], lam[3];
+  bonds3(x, r);
+  const int ca[3] = {0, 0, 1}, cb[3] = {1, 2, 2};
+#pragma unroll
+  for (int k = 0; k < 3; k++)
+    rhs[k] = -(r[k][0] * (v[ca[k]][0] - v[cb[k]][0]) + r[k][1] * (v[ca[k]][1] - v[cb[k]][1]) +
+               r[k][2] * (v[ca[k]][2] - v[cb[k]][2]));
+#pragma unroll
+  for (int k = 0; k < 3; k++) lam[k] = K.Mi[k][0] * rhs[0] + K.Mi[k][1] * rhs[1] + K.Mi[k][2] * rhs[2];
+  apply3(v, lam, r, im, 1.0);
+}
+
+__device__ __forceinline__ bool settle3(double x[SMA][3], const double xo[SMA][3], double v[SMA][3],
+                                        const RigidIso& K, double idt) {
+  if (!K.ok) return false;
+  const double wA = K.wA, wB = K.wB, rc = K.rc, ra = K.ra, rb = K.rb;
   double d[3], a1[3], b1[3], c1[3], b0[3], c0[3];
 #pragma unroll
   for (int k = 0; k < 3; k++) {
@@ -648,10 +710,10 @@ __device__ bool settle3(double x[SMA][3], const double xo[SMA][3], double v[SMA]
   const double a1z = dot3(ez, a1);
   const double b1x = dot3(ex, b1), b1y = dot3(ey, b1), b1z = dot3(ez, b1);
   const double c1x = dot3(ex, c1), c1y = dot3(ey, c1), c1z = dot3(ez, c1);
-  const double sphi = a1z / ra;
+  const double sphi = a1z * K.ira;
   if (!(fabs(sphi) < 1.0)) return false;
-  const double cphi = sqrt(1.0 - sphi * sphi);
-  const double spsi = (b1z - c1z) / (2.0 * rc * cphi);
+  const double cphi2 = 1.0 - sphi * sphi, icphi = rsqrt(cphi2), cphi = cphi2 * icphi;
+  const double spsi = (b1z - c1z) * K.irc2 * icphi;
   if (!(fabs(spsi) < 1.0)) return false;
   const double cpsi = sqrt(1.0 - spsi * spsi);
   // the canonical triangle tilted by phi and psi
@@ -664,7 +726,8 @@ __device__ bool settle3(double x[SMA][3], const double xo[SMA][3], double v[SMA]
   const double gamma = b0x * b1y - b0y * b1x + c0x * c1y - c0y * c1x;
   const double ab2 = alpha * alpha + beta * beta, disc = ab2 - gamma * gamma;
   if (!(disc >= 0.0 && ab2 > 0.0)) return false;
-  const double sth = (alpha * gamma - beta * sqrt(disc)) / ab2;
+  const double iab2 = 1.0 / ab2;  // (beside the square root)
+  const double sth = (alpha * gamma - beta * sqrt(disc)) * iab2;
   const double cth = sqrt(1.0 - sth * sth);
   const double p[3][3] = {{-a2y * sth, a2y * cth, a2z},
                           {b2x * cth - b2y * sth, b2x * sth + b2y * cth, b2z},
@@ -714,7 +777,7 @@ __device__ __forceinline__ void drift_atom(const MolArgs& A, int g, double dt) {
                    A.tcm);
     if (A.kick) v += kick_dv(A, i) * im;
     const double xo = A.x[i];
-    A.xo[i] = xo;
+    if (A.xo) A.xo[i] = xo;
     A.x[i] = xo + dt * v + f * 0.5 * dt * dt * im;
     A.v[i] = v + f * 0.5 * dt * im;
 #pragma unroll
@@ -861,7 +924,13 @@ __device__ __forceinline__ void drift_molecule(const MolArgs& A, int t, const in
   if constexpr (W3)
 #pragma unroll
     for (int k = 0; k < 3; k++) L2v[k] = __ldg(&A.dss[m.z + k]);
+  // isosceles with equal masses at the base: SETTLE, else Newton steps
+  const bool iso = W3 && im[1] == im[2] && fabs(L2v[0] - L2v[1]) <= 1e-12 * L2v[0];
+  RigidIso K;
+  if constexpr (W3)
+    if (iso) rigid_iso(im, L2v, K);
   pdl_enter();
+  pdl_release(A.early);
   double x[SMA][3], xo[SMA][3], v[SMA][3], fh[SMA][3];
   // positions, velocities, the kick's level forces and the verlet step's
   // N0 force (as 0.5 dt f / m), all issued before any arithmetic
@@ -947,10 +1016,15 @@ __device__ __forceinline__ void drift_molecule(const MolArgs& A, int t, const in
     }
   }
   if constexpr (W3) {
-    // isosceles with equal masses at the base: SETTLE, else Newton steps
-    const bool iso = im[1] == im[2] && fabs(L2v[0] - L2v[1]) <= 1e-12 * L2v[0];
-    if (!(iso ? settle3(x, xo, v, im, L2v, A.idt) : shake3(x, xo, v, im, L2v, dt, A.tol))) atomicOr(A.flag, 1);
-    if (!rattle3(x, v, im)) atomicOr(A.flag, 1);
+    if (iso) {
+      if (settle3(x, xo, v, K, A.idt))
+        rattle_iso(x, v, im, K);
+      else
+        atomicOr(A.flag, 1);
+    } else {
+      if (!shake3(x, xo, v, im, L2v, dt, A.tol)) atomicOr(A.flag, 1);
+      if (!rattle3(x, v, im)) atomicOr(A.flag, 1);
+    }
   } else if constexpr (KIND == MK_STAR) {
     if (!shake_star_n(nc, x, xo, v, im, A.dss + m.z, A.idt, A.tol)) atomicOr(A.flag, 1);
     if (!rattle_star_n(nc, x, v, im)) atomicOr(A.flag, 1);
@@ -966,7 +1040,7 @@ __device__ __forceinline__ void drift_molecule(const MolArgs& A, int t, const in
 #pragma unroll
       for (int d = 0; d < 3; d++) {
         A.x[d * N + g] = x[a][d];
-        A.xo[d * N + g] = xo[a][d];
+        if (A.xo) A.xo[d * N + g] = xo[a][d];
         A.v[d * N + g] = v[a][d];
 #pragma unroll
         for (int l = 0; l < NLV; l++)
@@ -1022,6 +1096,7 @@ __global__ void k_drift(const MolArgs A) {
       drift_molecule<MK_GENERAL, TH>(A, t, m);
   } else if (t < A.nsm + A.ndg) {
     pdl_enter();
+    pdl_release(A.early);
     // a group of an unconstrained molecule: its atoms, then its centre
     const int gi = A.drift_groups[t - A.nsm];
     const int2 mg = A.gmeta[gi];
@@ -1029,9 +1104,11 @@ __global__ void k_drift(const MolArgs A) {
     if (A.groups) group_centre(A, gi);
   } else if (t < A.nsm + A.ndg + A.nda) {
     pdl_enter();
+    pdl_release(A.early);
     drift_atom<TH>(A, A.drift_atoms[t - A.nsm - A.ndg], dt);
   } else {
     pdl_enter();
+    pdl_release(A.early);
   }
 }
 
@@ -1728,7 +1805,7 @@ static MolArgs mol_args(orac_gpu_ctx* ctx, MdState& S, double dt) {
   A.drift_atoms = S.drift_atoms;
   A.sm_atoms = S.sm_atoms;
   A.x = S.x;
-  A.xo = S.xo;
+  A.xo = S.nbig ? S.xo : nullptr;  // the iterative solvers' old positions
   A.v = S.v;
   A.invm = S.invm;
   A.pm = S.pm;
@@ -1757,6 +1834,7 @@ static MolArgs mol_args(orac_gpu_ctx* ctx, MdState& S, double dt) {
   A.groups = 1;
   A.tol = 1e-12;
   A.flag = S.flag;
+  A.early = orac_early(ctx);
   return A;
 }
 
@@ -1946,7 +2024,7 @@ static int md_ferrf(orac_gpu_ctx* ctx, MdState& S, unsigned long long* f, bool e
 // one shell's pair forces into its level accumulator (zeroed by the
 // preceding drift, or here when `zero`)
 static int md_shell_pair(orac_gpu_ctx* ctx, MdState& S, char sh, int lvl, bool zero, double* e, bool energy,
-                         bool no_next = false) {
+                         bool no_next = false, int more_flags = 0) {
   unsigned long long* f = S.ffix[lvl];
   if (zero) CK(cudaMemsetAsync(f, 0, sizeof(unsigned long long) * 3 * ctx->N, ctx->stream));
   // along a schedule force_alchemy's dwrk, U(lambda) - U(lambda0) over the
@@ -1959,7 +2037,7 @@ static int md_shell_pair(orac_gpu_ctx* ctx, MdState& S, char sh, int lvl, bool z
     CK(cudaMemsetAsync(pend, 0, sizeof(double), ctx->stream));
     ctx->pair_dwrk = pend;
   }
-  const int flags = SH_PREPPED | SH_FIXED_OUT | (energy ? SH_ENERGY : 0) | (no_next ? SH_NO_NEXT : 0);
+  const int flags = SH_PREPPED | SH_FIXED_OUT | (energy ? SH_ENERGY : 0) | (no_next ? SH_NO_NEXT : 0) | more_flags;
   const int rc0 = shell_run_r(ctx, sh, ctx->sh, ctx->d_xyz, ctx->d_grp, ctx->d_mol, reinterpret_cast<double*>(f),
                               energy ? e : nullptr, nullptr, flags);
   ctx->pair_dwrk = nullptr;
@@ -2216,7 +2294,14 @@ static int md_step(orac_gpu_ctx* ctx, MdState& S, bool update, bool energy) {
         if (int rc = md_pairs_n1(ctx, S, e_now, false)) return rc;
       if (int rc = ne_lambda_launch(ctx, per[LM])) return rc;
     }
-    if (side) {
+    // a substep of the innermost level alone has nothing to run beside its
+    // bonded terms: they follow the drift on the same stream, which spares
+    // the events' full dependencies (a kernel behind an event started 3 us
+    // after the one before it, one behind it in the stream 1 us)
+    const bool n0_only = S.has_n0 && !due_n1 && !due_m;
+    if (n0_only) {
+      if (int rc = md_bonded(ctx, S, true, false, e_now)) return rc;
+    } else if (side) {
       if (int rc = sd.fork()) return rc;
       if (int rc = sd.run([&]() -> int {
             if (int r2 = md_bonded(ctx, S, S.has_n0, due_n1, e_now)) return r2;
@@ -2245,7 +2330,12 @@ static int md_step(orac_gpu_ctx* ctx, MdState& S, bool update, bool energy) {
         return rc;
     }
     if (due_m) {
-      if (int rc = md_shell_pair(ctx, S, 'm', LM, false, S.e, e_now)) return rc;
+      // the M list is at least two kernels old here (the drift is between).
+      // The next kernel is released early unless it is another shell, whose
+      // waiting blocks would keep the SPME kernels out of the SMs
+      if (int rc = md_shell_pair(ctx, S, 'm', LM, false, S.e, e_now, false,
+                                 SH_LIST_OLD | (due_l ? 0 : SH_RELEASE)))
+        return rc;
       if (int rc = md_alch_m(ctx, S, e_now)) return rc;  // only without N1 pairs (else with them)
     }
     if (due_l && !split3)
@@ -2264,7 +2354,7 @@ static int md_step(orac_gpu_ctx* ctx, MdState& S, bool update, bool energy) {
     // the N1 level's pair terms beside the bonded kernel on the side stream
     if (due_n1 && !ne_m)
       if (int rc = md_pairs_n1(ctx, S, e_now, due_m)) return rc;
-    if (side)
+    if (side && !n0_only)
       if (int rc = sd.join()) return rc;
     if (ne_m) {
       // the M step's work, then the terms evaluated here become the held
@@ -2620,6 +2710,28 @@ int orac_gpu_md_setup(orac_gpu_ctx* ctx, const double* x, const double* y, const
       }
       if (!any) m.w |= NOINTRA;
     }
+  }
+  {
+    // molecules and clusters of one kind together, the general solver's first,
+    // then the stars by falling number of constraints, then the rigid
+    // triangles: a warp whose lanes hold different kinds runs each of their
+    // solvers in turn (the protein's clusters of 1, 2 and 3 hydrogens come
+    // mixed along its chain)
+    auto kind = [](const int4& m) {
+      const int nc = m.w & 0xff;
+      return (m.w & MOL3) ? 8 : ((m.w & STAR) ? 4 + SMC - nc : SMC - nc);
+    };
+    std::vector<int> ord(sm.size());
+    for (size_t q = 0; q < ord.size(); q++) ord[q] = (int)q;
+    std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) { return kind(sm[a]) < kind(sm[b]); });
+    std::vector<int4> sm2(sm.size());
+    std::vector<int2> smg2(sm.size());
+    for (size_t q = 0; q < ord.size(); q++) {
+      sm2[q] = sm[ord[q]];
+      smg2[q] = smg[ord[q]];
+    }
+    sm.swap(sm2);
+    smg.swap(smg2);
   }
   S.nsm = (int)sm.size();
   S.nfree = (int)fa.size();
