@@ -277,10 +277,15 @@ int orac_gpu_destroy(orac_gpu_ctx* ctx) {
                   ctx->d_gmol, ctx->d_amassinf, ctx->d_lj, ctx->d_ljd, ctx->d_exoff, ctx->d_exj, ctx->d_exrange, ctx->d_xyz, ctx->d_grp,
                   ctx->d_mol, ctx->d_gpos, ctx->d_aoff, ctx->d_ffix, ctx->d_acc, ctx->d_fout, ctx->d_red,
                   ctx->d_scan_tmp, ctx->d_total, ctx->d_flag, ctx->d_cell_of, ctx->d_cell_cnt, ctx->d_cell_start,
-                  ctx->d_cell_grp, ctx->d_stencil, ctx->pme.tw1, ctx->pme.tw2, ctx->pme.tw3, ctx->pme.bsp1,
-                  ctx->pme.bsp2, ctx->pme.bsp3, ctx->pme.qfix, ctx->pme.cgrid, ctx->pme.rgrid, ctx->pme.theta};
+                  ctx->d_cell_grp, ctx->d_stencil};
   for (void* p : ptrs)
     if (p) dev_free(ctx, p);
+  for (PmePlan* P : {&ctx->pme, &ctx->pme_call}) {
+    void* pp[] = {P->tw1,  P->tw2,   P->tw3,   P->bsp1,   P->bsp2, P->bsp3,
+                  P->qfix, P->cgrid, P->rgrid, P->cgsave, P->theta};
+    for (void* p : pp)
+      if (p) dev_free(ctx, p);
+  }
   void* aps[] = {ctx->api.cart, ctx->api.eout, ctx->api.ipairs, ctx->api.itype, ctx->api.t12,
                  ctx->api.t6,   ctx->api.ss,   ctx->api.e4,     ctx->api.q};
   for (void* p : aps)

@@ -428,8 +428,9 @@ struct orac_gpu_ctx {
   double* d_xtra = nullptr;  // [8] variant outputs of the last shell evaluation
   const double* pme_q() const { return variant == VAR_ALCH && d_qc ? d_qc : d_aqd; }
 
-  // PME
-  PmePlan pme;
+  // PME: the plan of the context's own grid (orac_gpu_set_ewald), and the
+  // last one that orac_gpu_do_pmesh_kspace was called with
+  PmePlan pme, pme_call;
 
   // measurement: work counters of the pair kernel and CUDA events around
   // its launches (recorded into captured graphs as event nodes)

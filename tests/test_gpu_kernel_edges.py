@@ -130,3 +130,32 @@ def test_plane_fft_grids(nfft, order):
     assert abs(eg - er) <= 1e-6 * abs(er)
     assert np.linalg.norm(vg - np.asarray(vr).reshape(3, 3)) <= 1e-5 * np.linalg.norm(vr)
     g.close()
+
+
+def test_plan_of_a_call_with_its_own_grid():
+    """Calls with their own grids leave the context's grid and results as they
+    are, and keep one plan's memory."""
+    from orac_b200.engine import Engine
+
+    s = systems.water_box(nwat=216, box=18.8, lattice=6, nfft=(20, 20, 20))
+    s.ncell = None
+    s.shells = small_shells()
+    g = Engine(s.copy())
+    F0, e0, _ = g.fft_pme()
+    r = s.cartesian()
+    a = (r[0], r[1], r[2], s.charge, 0.5 * s.oc.T, s.volume, s.alphal)
+    own = g.do_pmesh_kspace(*a, s.order, s.nfft)
+    A = g.do_pmesh_kspace(*a, 4, (24, 25, 27))
+    size = g.footprint()
+    B = g.do_pmesh_kspace(*a, 6, (20, 21, 18))
+    A2 = g.do_pmesh_kspace(*a, 4, (24, 25, 27))
+    assert g.footprint() == size
+    assert np.array_equal(A[0], A2[0]) and not np.array_equal(A[0], B[0])
+    assert rel_rms(own[0], F0) <= 1e-12 and abs(own[1] - e0) <= 1e-12 * abs(e0)
+    F1, e1, _ = g.fft_pme()
+    assert np.array_equal(F0, F1)
+    with pytest.raises(Exception):
+        g.do_pmesh_kspace(*a, 4, (22, 20, 20))  # 11 is no factor
+    F2, _, _ = g.fft_pme()
+    assert np.array_equal(F0, F2)
+    g.close()
