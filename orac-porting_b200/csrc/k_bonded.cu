@@ -35,6 +35,7 @@ struct BondedArgs {
   unsigned long long* ffix;   // [3N] fixed-point output
   unsigned long long* ffix_t; // [3N] fixed-point output of the proper torsions (their own r-RESPA level)
   double* e;                  // [8] (bond, bend, tors, itors) x (slt, slv), or null
+  int early;                  // pdl_release
 };
 
 template <bool TORS = false>
@@ -175,6 +176,7 @@ __device__ __forceinline__ void eadd(double* e, int type, double v) {
 
 __global__ void k_bonded(const BondedArgs A) {
   pdl_enter();
+  pdl_release(A.early);
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   double e[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   if ((A.mask & BK_BOND) && t < A.nb) {
@@ -378,6 +380,7 @@ int bonded_launch(orac_gpu_ctx* ctx, int mask, const double* d_x, double* d_f, u
   if (n == 0) return ORAC_OK;
   // 64 threads a block: the terms of one launch spread over four times the
   // SMs (each thread's FP64 chain sets the time, not the issue rate)
+  A.early = orac_early(ctx);
   orac_launch(k_bonded, (n + 63) / 64, 64, 0, ctx->stream, A);
   CKL();
   return ORAC_OK;

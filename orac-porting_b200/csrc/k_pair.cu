@@ -293,6 +293,7 @@ __global__ void __launch_bounds__(warps_per_block(MG) * 32, MINB) k_pair(const P
   __shared__ float4 s_ai[NQ][MG];
   __shared__ int s_ti[NQ][MG];  // the i atom's row of the LJ tables (type * ntype)
   __shared__ float s_pm[NQ][MG];
+  __shared__ double4 s_gi[NQ];
   __shared__ double s_qd[NQ][EN ? MG : 1];
   __shared__ int s_fi[NQ][VAR != VAR_STD ? MG : 1];
   __shared__ float2 s_sf[NQ][ALCH ? MG : 1];
@@ -361,7 +362,7 @@ __global__ void __launch_bounds__(warps_per_block(MG) * 32, MINB) k_pair(const P
   // and shuffles stay convergent
   {
     const int ifirst = mi.x, ni = mi.y & 15, typei = (mi.y >> 4) & 15, ljmi = (mi.y >> 8) & 0xff;
-    const double4 gi = gvalid ? A.gpos[i] : make_double4(0.0, 0.0, 0.0, 0.0);
+    if (sl == 0) s_gi[q] = gvalid ? A.gpos[i] : make_double4(0.0, 0.0, 0.0, 0.0);
     int mmax = m;
     if (SEG == 2) mmax = max(mmax, __shfl_xor_sync(FULL, m, 16));
     if (sl < MG) {  // (slots beyond the group's atoms: zeros, type 0)
@@ -401,6 +402,7 @@ __global__ void __launch_bounds__(warps_per_block(MG) * 32, MINB) k_pair(const P
       if (valid) {
         const double4 gj = A.gpos[j];
         mj = A.gmeta[j];
+        const double4 gi = s_gi[q];
         double dx = gi.x - gj.x, dy = gi.y - gj.y, dz = gi.z - gj.z;
         imx = 2.0 * round(0.5 * dx);
         imy = 2.0 * round(0.5 * dy);

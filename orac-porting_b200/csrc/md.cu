@@ -925,6 +925,16 @@ __device__ __forceinline__ void drift_molecule(const MolArgs& A, int t, const in
 #pragma unroll
     for (int k = 0; k < 3; k++) L2v[k] = __ldg(&A.dss[m.z + k]);
   // isosceles with equal masses at the base: SETTLE, else Newton steps
+  double ms[TH ? SMA : 1], iMs = 0.0;  // masses, and the molecule's inverse mass
+  if constexpr (TH) {
+    double M = 0.0;
+#pragma unroll
+    for (int a = 0; a < SMA; a++) {
+      ms[a] = a < na ? 1.0 / im[a] : 0.0;
+      M += ms[a];
+    }
+    iMs = 1.0 / M;
+  }
   const bool iso = W3 && im[1] == im[2] && fabs(L2v[0] - L2v[1]) <= 1e-12 * L2v[0];
   RigidIso K;
   if constexpr (W3)
@@ -956,12 +966,8 @@ __device__ __forceinline__ void drift_molecule(const MolArgs& A, int t, const in
     const bool big = (m.w & CLUSTER) != 0;
     const int p = big ? A.abm[gat[0]] : 0;
     const double sc = A.th->s[0], sk = A.th->s[A.tcls[gat[0]]];
-    double M = 0.0;
-#pragma unroll
-    for (int a = 0; a < SMA; a++)
-      if (a < na) M += 1.0 / im[a];
     double V[3], F[3];
-    const double iM = big ? 1.0 / A.bmass[p] : 1.0 / M;
+    const double iM = big ? 1.0 / A.bmass[p] : iMs;
 #pragma unroll
     for (int d = 0; d < 3; d++) {
       if (big) {
@@ -972,10 +978,10 @@ __device__ __forceinline__ void drift_molecule(const MolArgs& A, int t, const in
 #pragma unroll
         for (int a = 0; a < SMA; a++)
           if (a < na) {
-            tv += v[a][d] / im[a];
+            tv += v[a][d] * ms[a];
             tf += fixd(A.fk[LM][d * N + gat[a]]);
           }
-        V[d] = tv / M;
+        V[d] = tv * iMs;
         F[d] = tf;
       }
     }
@@ -1116,6 +1122,7 @@ __global__ void k_drift(const MolArgs A) {
 // molecules, after their iterative SHAKE
 __global__ void k_free_groups(const MolArgs A) {
   pdl_enter();
+  pdl_release(A.early);
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= A.nfreeg) return;
   group_centre(A, A.free_groups[t]);
@@ -1302,6 +1309,7 @@ constexpr int TS_BLOCK = 64;
 constexpr int TH_CHUNK = 64;
 
 struct ThermoArgs {
+  int early;  // pdl_release
   int N, nsm, nfree, nbm;
   const int4* sm;
   const int2* cloc;
@@ -1341,6 +1349,7 @@ __device__ __forceinline__ double msv(const ThermoArgs& A, int p, int j) { retur
 __global__ void __launch_bounds__(TS_BLOCK) k_mol_sums(const ThermoArgs A) {
   const int4 c = __ldg(&A.bchunk[blockIdx.x]);
   pdl_enter();
+  pdl_release(A.early);
   const int N = A.N;
   unsigned long long s[TH_NS];
 #pragma unroll
@@ -1423,9 +1432,19 @@ __device__ __forceinline__ void thermo_entry(const ThermoArgs& A, const int4 m, 
   }
   const int c = __ldg(&A.cls[gat[0]]);
   const int p = big ? __ldg(&A.abm[gat[0]]) : -1;
+  // masses and the molecule's, before the wait: a division of doubles is a
+  // chain of some 30 instructions, and 45 of them by inverse masses were
+  // most of this pass (20.4 us a launch for 3,000 waters)
+  double ms[SMA], M = 0.0;
+#pragma unroll
+  for (int a = 0; a < SMA; a++) {
+    ms[a] = a < na ? 1.0 / im[a] : 0.0;
+    M += ms[a];
+  }
+  const double iMs = 1.0 / M;
   pdl_enter();
+  pdl_release(A.early);
   double x[SMA][3], v[SMA][3];
-  double M = 0.0;
 #pragma unroll
   for (int a = 0; a < SMA; a++) {
 #pragma unroll
@@ -1433,7 +1452,6 @@ __device__ __forceinline__ void thermo_entry(const ThermoArgs& A, const int4 m, 
       x[a][d] = a < na ? A.x[d * N + gat[a]] : 0.0;
       v[a][d] = a < na ? A.v[d * N + gat[a]] : 0.0;
     }
-    if (a < na) M += 1.0 / im[a];
   }
   const double sc = A.th->s[0], sk = A.th->s[c];
   // centre-of-mass velocity and M force of a small molecule from its atoms
@@ -1443,8 +1461,8 @@ __device__ __forceinline__ void thermo_entry(const ThermoArgs& A, const int4 m, 
       double t = 0.0;
 #pragma unroll
       for (int a = 0; a < SMA; a++)
-        if (a < na) t += v[a][d] / im[a];
-      V[d] = t / M;
+        if (a < na) t += v[a][d] * ms[a];
+      V[d] = t * iMs;
     }
   };
   auto fsum = [&](double F[3]) {
@@ -1466,7 +1484,7 @@ __device__ __forceinline__ void thermo_entry(const ThermoArgs& A, const int4 m, 
         double t = 0.0;
 #pragma unroll
         for (int d = 0; d < 3; d++) t += (v[a][d] - V[d]) * (v[a][d] - V[d]);
-        u2 += t / im[a];
+        u2 += t * ms[a];
       }
     k[c] += u2;
     if (!big) k[0] += M * (V[0] * V[0] + V[1] * V[1] + V[2] * V[2]);
@@ -1481,7 +1499,8 @@ __device__ __forceinline__ void thermo_entry(const ThermoArgs& A, const int4 m, 
         if (a < na)
 #pragma unroll
           for (int d = 0; d < 3; d++)
-            v[a][d] += (A.c0 * fixf(A.f[LN0], d * N + gat[a]) + A.c1 * fixf(A.f[LN1], d * N + gat[a])) * im[a];
+            if (!(m.w & NOINTRA))
+              v[a][d] += (A.c0 * fixf(A.f[LN0], d * N + gat[a]) + A.c1 * fixf(A.f[LN1], d * N + gat[a])) * im[a];
       double Va[3], F[3];
       if (big) {
 #pragma unroll
@@ -1493,7 +1512,7 @@ __device__ __forceinline__ void thermo_entry(const ThermoArgs& A, const int4 m, 
         com(Va);
         fsum(F);
       }
-      const double iM = big ? B.iM : 1.0 / M;
+      const double iM = big ? B.iM : iMs;
 #pragma unroll
       for (int a = 0; a < SMA; a++)
         if (a < na)
@@ -1538,16 +1557,6 @@ __device__ __forceinline__ void thermo_entry(const ThermoArgs& A, const int4 m, 
       for (int d = 0; d < 3; d++) A.v[d * N + gat[a]] = v[a][d];
 }
 
-// correc_etap (src/correc_etap.f) with tto from comp_thermos_forces
-__device__ __forceinline__ void th_etap(ThermoDev& T, const double K[3]) {
-  for (int k = 0; k < 3; k++) {
-    if (fabs(T.q[k]) > 1.0e-7)
-      T.etap[k] += T.tm4 * (K[k] - T.ndfkt[k]) / T.q[k];
-    else
-      T.etap[k] = 0.0;
-  }
-}
-
 // Threads [0, nsm) take one small molecule or constraint cluster each,
 // [nsm, nsm + nfree) one atom outside them, the next nbm one molecule
 // outside the small ones (its centre-of-mass terms).  Each block leaves its
@@ -1574,6 +1583,7 @@ __global__ void __launch_bounds__(TH_BLOCK) k_thermo(const ThermoArgs A) {
     const int c = __ldg(&A.cls[g]);
     const int p = __ldg(&A.abm[g]);
     pdl_enter();
+    pdl_release(A.early);
     const double sc = A.th->s[0], sk = A.th->s[c];
     double v[3];
 #pragma unroll
@@ -1603,6 +1613,7 @@ __global__ void __launch_bounds__(TH_BLOCK) k_thermo(const ThermoArgs A) {
     for (int d = 0; d < 3; d++) A.v[d * N + g] = v[d];
   } else if (t < A.nsm + A.nfree + A.nbm) {
     pdl_enter();
+    pdl_release(A.early);
     {
       const int p = t - A.nsm - A.nfree;
       BigStages B;
@@ -1615,6 +1626,7 @@ __global__ void __launch_bounds__(TH_BLOCK) k_thermo(const ThermoArgs A) {
     }
   } else {
     pdl_enter();
+    pdl_release(A.early);
   }
   __shared__ double red[6][TH_BLOCK / 32];
   __shared__ bool last;
@@ -1641,6 +1653,11 @@ __global__ void __launch_bounds__(TH_BLOCK) k_thermo(const ThermoArgs A) {
   // the blocks' sums: lane l adds blocks l, l + 32, ... in order, then a
   // fixed butterfly over the lanes (the same result at every run)
   const volatile double* P = A.part;
+  // lane k moves thermostat k, its state read beside the sums
+  ThermoDev& T = *A.th;
+  const int k = threadIdx.x < 3 ? (int)threadIdx.x : 0;
+  double eta = T.eta[k], etap = T.etap[k];
+  const double q = T.q[k], ndfkt = T.ndfkt[k], tm = T.tm, tm4 = T.tm4;
   double K[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   if (threadIdx.x < 32)
     for (unsigned b = threadIdx.x; b < gridDim.x; b += 32)
@@ -1649,20 +1666,21 @@ __global__ void __launch_bounds__(TH_BLOCK) k_thermo(const ThermoArgs A) {
 #pragma unroll
   for (int j = 0; j < 6; j++)
     for (int o = 16; o > 0; o >>= 1) K[j] += __shfl_xor_sync(0xffffffffu, K[j], o);
-  if (threadIdx.x != 0) return;
-  const double K1[3] = {K[0], K[1], K[2]}, K2[3] = {K[3], K[4], K[5]};
-  ThermoDev& T = *A.th;
+  if (threadIdx.x >= 3) return;
+  // correc_etap twice (src/correc_etap.f) with tto from comp_thermos_forces
+  auto move = [&](double Kk) {
+    const double d = tm4 * (Kk - ndfkt) / q;
+    etap = fabs(q) > 1.0e-7 ? etap + d + d : 0.0;
+  };
   if (A.end) {
-    for (int k = 0; k < 3; k++) T.eta[k] += T.tm * T.etap[k];
-    th_etap(T, K1);
-    th_etap(T, K1);
+    eta += tm * etap;
+    move(k == 0 ? K[0] : (k == 1 ? K[1] : K[2]));
   }
-  if (A.k2) {
-    th_etap(T, K2);
-    th_etap(T, K2);
-  }
-  for (int k = 0; k < 3; k++) T.s[k] = exp(-T.tm4 * T.etap[k]);
-  T.count = 0;
+  if (A.k2) move(k == 0 ? K[3] : (k == 1 ? K[4] : K[5]));
+  T.eta[k] = eta;
+  T.etap[k] = etap;
+  T.s[k] = exp(-tm4 * etap);
+  if (k == 0) T.count = 0;
 }
 
 }  // namespace
@@ -1981,6 +1999,7 @@ static int md_thermo(orac_gpu_ctx* ctx, MdState& S, bool end, bool k2, double c0
   A.th = S.th;
   A.part = S.tpart;
   A.flag = S.flag;
+  A.early = orac_early(ctx);
   int slot = -1;
   if (int rc = prof_begin(ctx, &slot, PROF_DRIFT)) return rc;
   A.lvmask = (c0 != 0.0 && S.ffix[LN0] ? 1 : 0) | (c1 != 0.0 && S.ffix[LN1] ? 2 : 0) | 4 | (cl != 0.0 ? 8 : 0) |
