@@ -86,7 +86,7 @@ struct AlchDyn {
 struct GList {
   int* off = nullptr;   // [ngrp] row starts, in any order
   int* cnt = nullptr;   // [ngrp]
-  int* j = nullptr;     // [cap] partner group, 0-based; a pair is in one of the two rows
+  int* j = nullptr;     // [cap] partner group, 0-based, > row group
   unsigned long long* mask = nullptr;  // [cap] skipped atom pairs, bit a*8+b
   int64_t cap = 0;
   int64_t npairs = 0;   // host copy, updated when read back

@@ -5,7 +5,7 @@
 // ORAC bins group centres into ncx*ncy*ncz cells and, for every group n,
 // scans a precomputed stencil of cells keeping partners l > n whose
 // minimum-image centre distance is below rcut.  Here, where a pair is kept
-// once too, in one of the two groups' rows (keeps):
+// once too:
 //   k_cell_assign   cell of every group (ORAC's floor/wrap formula, FP64)
 //   k_scan          exclusive prefix sum (one block; lists are rebuilt every
 //                   few steps, so one block is enough)
@@ -138,26 +138,16 @@ struct ListArgs {
   int* flag;                  // bit 1 set where a row finds no room (null: not)
 };
 
-// Which of two groups keeps their pair in its row.  ORAC: the lower index.
-// Here: the one that has the other within half of the index circle ahead of
-// it, which is the lower index except across the circle's seam.  By plain
-// index the rows of a box's first groups hold the neighbours through the
-// periodic faces and those of its last ones none, and a pair kernel, with a
-// warp or half a warp a row, waits for the longest rows (3,000 waters, M list:
-// 0 to 35 entries, mean 12).  The rule depends on indices alone, so a list
-// built again gives every pair the same two roles and bitwise the same forces;
-// by turns of the parity the rows balance too, but hold both sides of a
-// group's surroundings, and the kernels of the longer lists read half as much
-// again (L shell 17.9 against 15.1 us).
-__device__ __forceinline__ bool keeps(int i, int l, int G) {
-  int d = l - i;
-  if (d < 0) d += G;
-  return d != 0 && (2 * d < G || (2 * d == G && i < l));
-}
-
+// A pair is kept by the group of lower index, as in ORAC.  Rules that balance
+// the rows (the first groups' hold all neighbours through the periodic faces,
+// the last ones' none) were measured and dropped: by the parity of the index
+// difference a row holds both sides of its group's surroundings and the longer
+// lists' kernels read more (L shell 17.9 against 15.1 us for 3,000 waters);
+// within half the index circle ahead gave 0 to 1% on 9,000 and 22,700 atoms
+// and cost 2% on 81,000, on replicas and on single evaluations.
 __device__ __forceinline__ bool pair_in(const ListArgs& A, double xi, double yi,
                                         double zi, int i, int l) {
-  if (!keeps(i, l, A.G)) return false;
+  if (l <= i) return false;
   double dx = xi - A.grp[l], dy = yi - A.grp[A.G + l], dz = zi - A.grp[2 * A.G + l];
   dx -= 2.0 * round(0.5 * dx);  // pbc.h: anint(0.5 x)
   dy -= 2.0 * round(0.5 * dy);
@@ -173,14 +163,6 @@ __device__ __forceinline__ bool pair_in(const ListArgs& A, double xi, double yi,
 // are both >= massinfty (src/force.f:374-388, 486-489).
 __device__ unsigned long long pair_mask(const ListArgs& A, int i, int l) {
   if (A.gmol[i] != A.gmol[l]) return 0ull;
-  // mapnl lists each exclusion at the atom of lower index, and the fixed-mass
-  // rule is that group's: evaluated from there, and turned for the higher one
-  const bool turn = l < i;
-  if (turn) {
-    const int k = i;
-    i = l;
-    l = k;
-  }
   const int2 mi = A.gmeta[i], ml = A.gmeta[l];
   const int i0 = mi.x, ni = mi.y & 0xff, l0 = ml.x, nl = ml.y & 0xff;
   // most groups of a large molecule lie beyond its excluded partners
@@ -199,11 +181,6 @@ __device__ unsigned long long pair_mask(const ListArgs& A, int i, int l) {
     if (any && A.massinf[i0 + a])
       for (int b = 0; b < nl; b++)
         if (A.massinf[l0 + b]) m |= 1ull << (a * 8 + b);
-  }
-  if (turn && m) {
-    unsigned long long r = 0ull;
-    for (int k = 0; k < 64; k++) r |= ((m >> k) & 1ull) << ((k & 7) * 8 + (k >> 3));
-    m = r;
   }
   return m;
 }

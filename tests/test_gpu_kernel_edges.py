@@ -1,7 +1,6 @@
 """GPU kernels at the sizes where their tiles end, against the FP64 oracle:
 the pair kernel's rows (one group pair to several passes, groups of up to 3,
-4 and 8 atoms, half and whole warps a row) and the seam of the list's
-ownership rule, the plane FFT (odd axes, one x line left over, planes too
+4 and 8 atoms, half and whole warps a row), the plane FFT (odd axes, one x line left over, planes too
 large for shared memory) and the plan kept for calls that bring their own
 grid.  Tolerances as in the other parity tests: forces relative RMS <= 1e-5
 (FP32 pair and spline arithmetic), energies 1e-6 of the terms' magnitudes.
@@ -25,9 +24,8 @@ def small_shells():
 
 
 @pytest.mark.parametrize("nwat", [2, 3, 4, 17, 64, 65])
-def test_rows_and_ownership_of_few_groups(nwat):
-    """All-pairs lists of 2 to 65 groups: rows of no entry to several passes,
-    and for even counts the pairs half the index circle apart."""
+def test_rows_of_few_groups(nwat):
+    """All-pairs lists of 2 to 65 groups: rows of no entry to several passes."""
     from orac_b200.engine import Engine
 
     s = systems.water_box(nwat=nwat, box=18.8, lattice=5, nfft=(20, 20, 20))
@@ -51,7 +49,7 @@ def test_rows_and_ownership_of_few_groups(nwat):
 @pytest.mark.parametrize("lanes", [(16, 16), (32, 32)])
 def test_group_sizes_and_lanes(group_size, lanes):
     """Chains cut in groups of 1 to 8 atoms in water: each build of the pair
-    kernel, with exclusion masks on both sides of the ownership rule."""
+    kernel, with exclusion masks."""
     from orac_b200.engine import Engine
 
     s = systems.solvated_chains(2100, 31, group_size=group_size)
