@@ -70,7 +70,10 @@ const char* orac_gpu_version(void);
  * 1-based into ecc12/ecc6 of length ntype*(ntype+1)/2).  mapnl is the serial
  * exclusion map built by mappa (src/mappa.f): for each atom i in order,
  * [n, j_1 .. j_n] with j > i.  pmass is the mass fraction of each atom in its
- * group (ORAC's pmass/gmass, src/redmss.f:15). */
+ * group (ORAC's pmass/gmass, src/redmss.f:15).  A later call replaces the
+ * topology: the lists and the MD state (orac_gpu_md_setup) are gone; bonded
+ * terms, intramolecular pairs and the REM or alchemy selection (with a
+ * schedule) stay where ntap is the same and are dropped where it is not. */
 int orac_gpu_set_topology(orac_gpu_ctx* ctx, int ntap, int ngrp, int nprot,
                           const int* grppt, const int* atomp, const int* atomg,
                           const int* ss_index, const double* chrge,

@@ -316,6 +316,7 @@ int orac_gpu_set_topology(orac_gpu_ctx* ctx, int ntap, int ngrp, int nprot, cons
                           const int* atomg, const int* ss_index, const double* chrge, const int* nbtype, int ntype,
                           const int* type_table, const double* ecc12, const double* ecc6, const double* mass,
                           const double* pmass, double massinfty, const int* mapnl, int64_t nmapnl) {
+  ParamGenBump bump(ctx);  // kernels capture these values: step graphs are re-captured
   if (!ctx) return ORAC_ERR_PARAM;
   if (ntap <= 0 || ngrp <= 0 || nprot <= 0 || ntype <= 0)
     return ctx_fail(ctx, ORAC_ERR_PARAM, "bad sizes ntap=%d ngrp=%d nprot=%d ntype=%d", ntap, ngrp, nprot, ntype);
@@ -338,7 +339,7 @@ int orac_gpu_set_topology(orac_gpu_ctx* ctx, int ntap, int ngrp, int nprot, cons
     maxg = n > maxg ? n : maxg;
     const int ss = ss_index[a0];
     if (ss != 1 && ss != 2) return ctx_fail(ctx, ORAC_ERR_PARAM, "ss_index of atom %d is %d", a0 + 1, ss);
-    gmeta[g] = make_int2(a0, n | (ss << 8));  // LJ-atom mask added below
+    gmeta[g] = make_int2(a0, n | (ss << 8));
     gmol[g] = atomp[a0] - 1;
     for (int a = a0; a <= a1; a++) {
       if (atomg[a] != g + 1) return ctx_fail(ctx, ORAC_ERR_PARAM, "atomg(%d) != %d", a + 1, g + 1);
@@ -401,6 +402,18 @@ int orac_gpu_set_topology(orac_gpu_ctx* ctx, int ntap, int ngrp, int nprot, cons
     }
     exoff[N] = (int)exj.size();
   }
+  // What an earlier topology left in the context.  The MD state and its step
+  // graphs hold that topology's arrays and group indices.  Terms and selections
+  // by atom stay where the number of atoms does (a caller may upload changed
+  // charges or parameters), and are dropped where it does not: their arrays
+  // have the earlier length.
+  const bool same_atoms = ctx->have_topo && N == ctx->N;
+  bump.arm();
+  if (ctx->md) {
+    CK(cudaStreamSynchronize(ctx->stream));
+    md_destroy(ctx);
+  }
+  ctx->have_topo = false;
   ctx->N = N;
   ctx->G = G;
   ctx->P = P;
@@ -415,8 +428,11 @@ int orac_gpu_set_topology(orac_gpu_ctx* ctx, int ntap, int ngrp, int nprot, cons
   }
   ctx->h_amol = amol;
   ctx->h_gmol = gmol;
-  ctx->h_intra_b.clear();  // bonded terms of an earlier topology no longer apply
-  ctx->h_intra_p.clear();
+  if (!same_atoms) {
+    ctx->h_intra_b.clear();
+    ctx->h_intra_p.clear();
+    bonded_free(ctx);
+  }
   ctx->h_charge.assign(chrge, chrge + N);
   ctx->h_mass.assign(mass, mass + N);
   ctx->h_ss.assign(ss_index, ss_index + N);
@@ -471,8 +487,16 @@ int orac_gpu_set_topology(orac_gpu_ctx* ctx, int ntap, int ngrp, int nprot, cons
   }
   ctx->lists[1].off = ctx->lists[0].off;
   ctx->lists[2].off = ctx->lists[0].off;
+  // solute and solvent by atom: read from h_ss again at the next use
+  dev_free(ctx, ctx->bd.ss);
+  ctx->bd.ss = nullptr;
+  dev_free(ctx, ctx->api.ss);
+  ctx->api.ss = nullptr;
+  if (int rc = variant_topology(ctx, same_atoms)) return rc;
+  if (dev_alloc(ctx, &ctx->d_gpair, G)) return ORAC_ERR_CUDA;
+  if (int rc = pair_meta_build(ctx)) return rc;
   ctx->have_topo = true;
-  return pair_meta_build(ctx);
+  return ORAC_OK;
 }
 
 int orac_gpu_set_ewald(orac_gpu_ctx* ctx, int clewld, double alphal, int order, int nfft1, int nfft2, int nfft3,

@@ -144,6 +144,34 @@ int alch_upload_tables(orac_gpu_ctx* ctx) {
   return ORAC_OK;
 }
 
+int variant_topology(orac_gpu_ctx* ctx, bool same_atoms) {
+  if (same_atoms) return ctx->h_vflag.empty() ? ORAC_OK : build_vflag(ctx);  // (fixed masses may differ)
+  ctx->variant = VAR_STD;
+  ctx->h_rem.clear();
+  ctx->h_ssal.clear();
+  ctx->h_softlj.clear();
+  ctx->h_vflag.clear();
+  ctx->ne.on = false;
+  ctx->nlistqq = -1;
+  ctx->q0_differs = false;
+  ctx->self_dudl = 0.0;
+  auto drop = [&](auto*& p) {
+    dev_free(ctx, p);
+    p = nullptr;
+  };
+  drop(ctx->d_vflag);
+  drop(ctx->d_soft);
+  drop(ctx->d_softd);
+  drop(ctx->d_qc);
+  drop(ctx->d_q0);
+  drop(ctx->d_dq);
+  drop(ctx->d_lam4);
+  drop(ctx->d_lam40);
+  drop(ctx->d_ne_dq);
+  drop(ctx->d_ne_alist);
+  drop(ctx->d_listqq);
+  return ORAC_OK;
+}
 
 int pair_meta_build(orac_gpu_ctx* ctx) {
   const bool alch = ctx->variant == VAR_ALCH, rem = ctx->variant == VAR_REM;
@@ -163,7 +191,6 @@ int pair_meta_build(orac_gpu_ctx* ctx) {
     }
     gm[g] = make_int4(first, y, (int)ty[0], (int)ty[1]);
   }
-  if (!ctx->d_gpair && dev_alloc(ctx, &ctx->d_gpair, gm.size())) return ORAC_ERR_CUDA;
   CK(cudaMemcpy(ctx->d_gpair, gm.data(), gm.size() * sizeof(int4), cudaMemcpyHostToDevice));
   return ORAC_OK;
 }
@@ -233,7 +260,7 @@ int alch_listqq_build(orac_gpu_ctx* ctx) {
 
 void variant_free(orac_gpu_ctx* ctx) {
   void* p[] = {ctx->d_vflag, ctx->d_soft, ctx->d_softd, ctx->d_qc, ctx->d_q0, ctx->d_xtra, ctx->d_dq,
-               ctx->d_lam4, ctx->d_listqq, ctx->d_remf, ctx->d_ad, ctx->d_lam40, ctx->d_ne, ctx->d_ne_alist};
+               ctx->d_lam4, ctx->d_listqq, ctx->d_remf, ctx->d_ad, ctx->d_lam40, ctx->d_ne, ctx->d_ne_alist, ctx->d_ne_dq};
   for (void* q : p)
     if (q) dev_free(ctx, q);
 }

@@ -472,7 +472,10 @@ int prof_collect(orac_gpu_ctx* ctx, int a, int b);
 void variant_fill(const orac_gpu_ctx* ctx, PairArgs* a);
 int variant_out_launch(orac_gpu_ctx* ctx, int forces_on);
 void variant_free(orac_gpu_ctx* ctx);
-// rebuild d_gpair after the topology or the variant changed
+// the REM or alchemy selection and the schedule after a topology call: kept
+// with the number of atoms, else dropped
+int variant_topology(orac_gpu_ctx* ctx, bool same_atoms);
+// fill d_gpair (set_topology sizes it) after the topology or the variant changed
 int pair_meta_build(orac_gpu_ctx* ctx);
 
 // ---------------------------------------------------------------- errors

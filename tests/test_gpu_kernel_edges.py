@@ -157,3 +157,75 @@ def test_plan_of_a_call_with_its_own_grid():
     F2, _, _ = g.fft_pme()
     assert np.array_equal(F0, F2)
     g.close()
+
+
+def _same_as_fresh(g, s, setup):
+    """Context g, given topology s after others, against a fresh context, bit for bit."""
+    from orac_b200.engine import Engine
+
+    f = Engine(s.copy())
+    setup(f)
+    f.update_lists()
+    g.update_lists()
+    for sh in "mlh":
+        Ff, ef, sf = f.shell(sh)
+        Fg, eg, sg = g.shell(sh)
+        assert np.abs(Ff).max() > 0 and np.array_equal(Fg, Ff), sh
+        # (energies and stress: FP64 sums of atomics, in any order)
+        assert np.allclose(g.ue6(eg), f.ue6(ef), rtol=1e-12, atol=1e-9)
+        assert np.linalg.norm(sg - sf) <= 1e-10 * np.linalg.norm(sf)
+    if s.has_intra():
+        assert rel_rms(g.intra_n1()[0], f.intra_n1()[0]) <= 1e-12
+    f.close()
+
+
+def test_topologies_one_after_another():
+    """One context that takes a small topology, a larger one, the larger one
+    with alchemy, a smaller one and its own again: what the earlier ones left
+    (group records, selections by atom, bonded terms, MD state) neither stays
+    in use nor sizes what follows."""
+    from orac_b200.engine import Engine
+    from orac_b200.lib import OracGpuError
+
+    def take(g, s):
+        g.s = s.copy()
+        g._upload()
+
+    def alch(e):
+        e.set_alchemy(e.s.ss_alchemy, 0.5, 0.5)
+        e.set_lambda(0.0, 0.3, 0.0, 0.6)
+
+    def rem(e):
+        e.set_rem(np.arange(e.s.ntap) % 5 == 0, 0, 0.7)
+
+    def none(e):
+        pass
+
+    small = systems.water_box(nwat=64, box=18.8, lattice=5, nfft=(20, 20, 20))
+    small.ncell = None
+    small.shells = small_shells()
+    chains = systems.solvated_chains(2100, 31)
+    ligand = systems.ligand_in_water(nlig=13, nwat=1000, box=31.3, nfft=(32, 32, 32))
+    ligand.ncell = (systems.linked_cells_for(31.3, ligand.shells),) * 3
+    g = Engine(small.copy())
+    rem(g)
+    _same_as_fresh(g, small, rem)
+    take(g, chains)  # larger: the selection by atom is gone
+    _same_as_fresh(g, chains, none)
+    g.md_setup(4.0, 2, 4, 6, "l")
+    g.md_run(1)
+    take(g, ligand)
+    with pytest.raises(OracGpuError, match="md_setup"):
+        g.md_run(1)
+    _same_as_fresh(g, ligand, none)
+    alch(g)
+    _same_as_fresh(g, ligand, alch)
+    take(g, ligand)  # the same number of atoms: the selection stays
+    _same_as_fresh(g, ligand, alch)
+    g.md_setup(4.0, 2, 4, 6, "l")
+    g.md_run(1)
+    take(g, small)
+    _same_as_fresh(g, small, none)
+    take(g, chains)
+    _same_as_fresh(g, chains, none)
+    g.close()
