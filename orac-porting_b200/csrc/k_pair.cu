@@ -519,14 +519,13 @@ __global__ void __launch_bounds__(warps_per_block(MG) * 32, MINB) k_pair(const P
             double pconf = 0.0, pcoul = 0.0, px0 = 0.0, px1 = 0.0, px2 = 0.0;
             // the straight path: every pair of the two groups without a branch,
             // so that the pairs' chains of dependent instructions overlap; pairs
-            // that are not to be evaluated take part at distance 1 with
-            // coefficients 0.  Three pairs share one test for LJ (in water only
-            // the oxygens have it).  Not for pairs of LJ alone (one in nine of
-            // water's) nor for groups with alchemical or fixed-mass atoms.
-            const bool straight = MG <= 4 && !A.lskip && !(ALCH && ((mi.y | me.y) & GM_SPECIAL));
+            // that are not to be evaluated take part with coefficients 0.  Three
+            // pairs share one test for LJ (in water only the oxygens have it).
+            // Not for pairs of LJ alone (one in nine of water's) nor for groups
+            // with alchemical or fixed-mass atoms.
+            bool straight = MG <= 4 && !A.lskip && !(ALCH && ((mi.y | me.y) & GM_SPECIAL));
             if constexpr (MG <= 4) {
               if (straight) {
-                npairs += __popc((unsigned)pb);
                 float4 ob[MG];
 #pragma unroll
                 for (int b = 0; b < MG; b++)
@@ -542,8 +541,7 @@ __global__ void __launch_bounds__(warps_per_block(MG) * 32, MINB) k_pair(const P
                     rx[a] = ad(ai.x, bx);
                     ry[a] = ad(ai.y, by);
                     rz[a] = ad(ai.z, bz);
-                    float r2 = fm(rz[a], rz[a], fm(ry[a], ry[a], mu(rx[a], rx[a])));
-                    r2 = on ? r2 : 1.f;
+                    const float r2 = fm(rz[a], rz[a], fm(ry[a], ry[a], mu(rx[a], rx[a])));
                     const float qq = on ? mu(ai.w, ob[b].w) : 0.f;
                     // 1/r from the hardware reciprocal square root, exp from ex2
                     // and an approximate reciprocal: a few ulp, far below the
@@ -611,6 +609,23 @@ __global__ void __launch_bounds__(warps_per_block(MG) * 32, MINB) k_pair(const P
                     gjy += fby;
                     gjz += fbz;
                   }
+                }
+                // V is no number where a coordinate is none or infinite (every pair's
+                // distance enters it, also of the pairs that are not to be evaluated,
+                // with coefficient 0), or where such a pair has no distance at all.
+                // Their forces would then be NaN too, and those of the slots beyond a
+                // group's atoms belong to other atoms or to none: the entry is
+                // evaluated pair by pair instead.
+                if (V == V) {
+                  npairs += __popc((unsigned)pb);
+                } else {
+                  straight = false;
+                  V = 0.f;
+                  gjx = gjy = gjz = 0.0;
+#pragma unroll
+                  for (int a = 0; a < MG; a++)
+#pragma unroll
+                    for (int c = 0; c < 3; c++) fi[a][c] = fj[a][c] = 0.f;
                 }
               }
             }
@@ -770,7 +785,8 @@ __global__ void __launch_bounds__(warps_per_block(MG) * 32, MINB) k_pair(const P
               if constexpr (MG <= 4) {
 #pragma unroll
                 for (int b = 0; b < MG; b++) {
-                  const float pm = b < nj ? A.apm[jf + b] : 0.f;
+                  if (b >= nj) continue;
+                  const float pm = A.apm[jf + b];
                   fj[b][0] = fm(-pm, sx, fj[b][0]);
                   fj[b][1] = fm(-pm, sy, fj[b][1]);
                   fj[b][2] = fm(-pm, sz, fj[b][2]);
@@ -798,7 +814,7 @@ __global__ void __launch_bounds__(warps_per_block(MG) * 32, MINB) k_pair(const P
             }
             if constexpr (MG <= 4) {
 #pragma unroll
-              for (int b = 0; b < MG; b++) {  // (zero beyond the group's atoms)
+              for (int b = 0; b < MG; b++) {  // (zero beyond the group's atoms, whatever the coordinates)
                 fix_add(A.ffix + jf + b, fj[b][0]);
                 fix_add(A.ffix + A.natom + jf + b, fj[b][1]);
                 fix_add(A.ffix + 2 * A.natom + jf + b, fj[b][2]);

@@ -229,3 +229,85 @@ def test_topologies_one_after_another():
     take(g, chains)
     _same_as_fresh(g, chains, none)
     g.close()
+
+
+def _shell_dev(g, sh, energies=False):
+    """Forces (3, N) of one shell through orac_gpu_mts_forces_dev."""
+    import torch
+
+    dev = torch.device("cuda", 0)
+    x, gr, mo = (torch.from_numpy(np.concatenate(a)).to(dev) for a in (
+        (g.xp0, g.yp0, g.zp0), (g.xpg, g.ypg, g.zpg), (g.xpcm, g.ypcm, g.zpcm)))
+    f = torch.zeros(3 * g.s.ntap, dtype=torch.float64, device=dev)
+    e = torch.zeros(8, dtype=torch.float64, device=dev)
+    torch.cuda.synchronize()
+    rc = g.lib.orac_gpu_mts_forces_dev(g.ctx, sh.encode(), x.data_ptr(), gr.data_ptr(), mo.data_ptr(), f.data_ptr(),
+                                       e.data_ptr() if energies else None, None)
+    assert rc == 0
+    torch.cuda.synchronize()
+    return f.cpu().numpy().reshape(3, -1)
+
+
+def _exclusions(s):
+    out, p = [[] for _ in range(s.ntap)], 0
+    for i in range(s.ntap):
+        for j in s.mapnl[p + 1:p + 1 + s.mapnl[p]]:
+            out[i].append(j - 1)
+            out[j - 1].append(i)
+        p += 1 + s.mapnl[p]
+    return out
+
+
+@pytest.mark.parametrize("group_size", [3, 4, 8])
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+@pytest.mark.parametrize("variant", ["std", "rem", "alchemy"])
+def test_a_coordinate_that_is_no_number(group_size, value, variant):
+    """An atom without coordinates spoils the forces of the groups in reach of
+    its own (an evaluated pair with it, or the S'V share), and nothing else:
+    not the atoms that follow a shorter group in the force array, not the
+    atoms whose only pair with it is excluded."""
+    from orac_b200.engine import Engine
+
+    s = systems.solvated_chains(2100, 31, group_size=group_size)
+    g = Engine(s.copy())
+    if variant == "rem":
+        g.set_rem(np.arange(s.ntap) % 5 == 0, 0, 0.7)
+    elif variant == "alchemy":
+        g.set_alchemy(np.where(np.arange(s.ntap) < 4, -2, 1), 0.5, 0.5)
+        g.set_lambda(0.0, 0.3, 0.0, 0.6)
+    g.update_lists()
+    sh = s.shells
+    first, last = s.grppt[:, 0] - 1, s.grppt[:, 1] - 1
+    excl = _exclusions(s)
+    size = last - first + 1
+    # atoms near the end of their group in a chain, and the last molecule's last
+    for a in (22, 23, s.ntap - 1):
+        grp = int(s.atomg[a]) - 1
+        d = np.stack([g.xpg - g.xpg[grp], g.ypg - g.ypg[grp], g.zpg - g.zpg[grp]])
+        r = np.linalg.norm(np.asarray(s.co) @ (d - 2.0 * np.round(0.5 * d)), axis=0)
+        far, masked = {}, []
+        for k, ro, to, ri in (("m", sh.rcutm, sh.rtolm, 0.0), ("l", sh.rcutl, sh.rtoll, sh.rcutm)):
+            near = (r < ro + to) & (r >= ri)
+            near[grp] = True
+            far[k] = ~np.repeat(near, size)
+        for b in excl[a]:  # in the unswitched band of the M shell
+            j = int(s.atomg[b]) - 1
+            if j != grp and r[j] < sh.rcutm:
+                masked.append(b)
+        clean = {k: [_shell_dev(g, k, e) for e in (False, True)] for k in "ml"}
+        keep = g.xp0
+        g.xp0 = keep.copy()
+        g.xp0[a] = value
+        for k in "ml":
+            for e in (False, True):
+                F = _shell_dev(g, k, e)
+                c = clean[k][e]
+                assert np.array_equal(F[:, far[k]], c[:, far[k]]), (k, a)
+                if k == "m":
+                    # an entry evaluated pair by pair rounds differently: a few
+                    # FP32 roundings of forces no larger than the largest
+                    assert np.abs(F - c)[:, masked].max(initial=0.0) <= 1e-6 * np.abs(c).max(), (k, a)
+        g.xp0 = keep
+        assert all(v.sum() > s.ntap // 2 for v in far.values())
+        assert masked or group_size == 8 or a == s.ntap - 1
+    g.close()
