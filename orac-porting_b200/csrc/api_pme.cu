@@ -64,7 +64,7 @@ struct PlanOfCall {
   bool swapped;
   PlanOfCall(orac_gpu_ctx* c, int n1, int n2, int n3, int order) : ctx(c) {
     const PmePlan& P = c->pme;
-    swapped = !(P.qfix && P.n1 == n1 && P.n2 == n2 && P.n3 == n3 && P.order == order);
+    swapped = !(P.ready && P.n1 == n1 && P.n2 == n2 && P.n3 == n3 && P.order == order);
     if (swapped) std::swap(c->pme, c->pme_call);
   }
   ~PlanOfCall() {

@@ -797,7 +797,8 @@ int pme_setup(orac_gpu_ctx* ctx, int n1, int n2, int n3, int order) {
   FftPlan f;
   if (make_plan(n1, &f) || make_plan(n2, &f) || make_plan(n3, &f))
     return ctx_fail(ctx, ORAC_ERR_PARAM, "PME grid %dx%dx%d: sizes must factor into 2, 3, 5, 7", n1, n2, n3);
-  if (P.n1 == n1 && P.n2 == n2 && P.n3 == n3 && P.order == order && P.qfix) return ORAC_OK;
+  if (P.ready && P.n1 == n1 && P.n2 == n2 && P.n3 == n3 && P.order == order) return ORAC_OK;
+  P.ready = false;  // until every allocation below has succeeded
   P.n1 = n1;
   P.n2 = n2;
   P.n3 = n3;
@@ -817,8 +818,10 @@ int pme_setup(orac_gpu_ctx* ctx, int n1, int n2, int n3, int order) {
     CK(cudaFuncSetAttribute(k_plane<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PLANE_SMEM_MAX));
   }
   const size_t ng = (size_t)n1 * n2 * n3;
-  if (dev_alloc(ctx, &P.qfix, ng) || dev_alloc(ctx, &P.rgrid, ng) || dev_alloc(ctx, &P.cgrid, (size_t)P.h1 * n2 * n3))
+  const size_t nc = (size_t)P.h1 * n2 * n3;
+  if (dev_alloc(ctx, &P.qfix, ng) || dev_alloc(ctx, &P.rgrid, ng) || dev_alloc(ctx, &P.cgrid, nc))
     return ORAC_ERR_CUDA;
+  P.ready = true;
   return ORAC_OK;
 }
 
@@ -827,7 +830,7 @@ int pme_run(orac_gpu_ctx* ctx, int natom, const double* d_cart, const double* d_
             unsigned long long* d_ffix, const double* d_dq, double* d_edq, float2* d_save,
             const float2* d_cross, bool sums) {
   PmePlan& P = ctx->pme;
-  if (!P.qfix) return ctx_fail(ctx, ORAC_ERR_STATE, "PME not set up");
+  if (!P.ready) return ctx_fail(ctx, ORAC_ERR_STATE, "PME not set up");
   const int n1 = P.n1, n2 = P.n2, n3 = P.n3, h1 = P.h1;
   CK(cudaMemsetAsync(P.qfix, 0, sizeof(unsigned long long) * (size_t)n1 * n2 * n3, ctx->stream));
   if (sums) CK(cudaMemsetAsync(d_eout, 0, sizeof(double) * 16, ctx->stream));
