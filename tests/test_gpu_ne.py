@@ -154,3 +154,50 @@ def test_f0_test4_work_matches_the_oracle_and_what_orac_printed():
     np.testing.assert_allclose(wg * units.KJMOL, d["wrk1"][0, 5], rtol=4e-3)
     g.close()
     o.close()
+
+
+def test_schedule_on_another_grid():
+    """A schedule's run set up on one SPME grid, then on a larger one in the
+    same context: the kept transformed grid of the work's reciprocal term has
+    the size of the grid in use, after orac_gpu_md_setup and within a run."""
+    s = systems.ligand_in_water(nlig=13, nwat=1000, box=31.3, nfft=(32, 32, 32))
+    s.ncell = (systems.linked_cells_for(31.3, s.shells),) * 3
+
+    def make(nfft):
+        t = s.copy()
+        t.nfft = nfft
+        g = Engine(t)
+        g.set_alchemy(s.ss_alchemy, 0.5, 0.5)
+        g.set_lambda(0.0, 0.0, 0.0, 0.0)
+        g.set_schedule(TIMES, LAMS["ladded"], LAMS["laddedq"], LAMS["lremoved"], LAMS["lremovedq"])
+        return g
+
+    def setup(g):
+        g.md_setup(SCHED["dt_h"], SCHED["lrespa"], SCHED["mrespa"], SCHED["nupdte"], SCHED["rshk"],
+                   n1respa=SCHED["n1respa"], n0respa=SCHED["n0respa"])
+
+    def grid(g, n):
+        rc = g.lib.orac_gpu_set_ewald(g.ctx, 1, s.alphal, s.order, *n, s.rkcut)
+        assert rc == 0
+
+    f = make((48, 45, 40))
+    setup(f)
+    f.md_run(2)
+    g = make((32, 32, 32))
+    setup(g)
+    g.md_run(2)
+    small = g.md_work()[0]
+    grid(g, (48, 45, 40))
+    setup(g)
+    g.md_run(2)
+    assert abs(g.md_work()[0] - f.md_work()[0]) <= 1e-9 * abs(f.md_work()[0])
+    assert np.array_equal(g.md_state()[0], f.md_state()[0])
+    # (the two grids' SPME errors: a few 1e-4 of a work that the direct sum dominates)
+    assert abs(small - f.md_work()[0]) <= 5e-3 * abs(small)
+    # a larger grid in the middle of a run
+    f.md_run(2)
+    grid(g, (60, 54, 56))
+    g.md_run(2)
+    assert abs(g.md_work()[0] - f.md_work()[0]) <= 5e-3 * abs(f.md_work()[0])
+    f.close()
+    g.close()
