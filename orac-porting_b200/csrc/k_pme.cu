@@ -608,7 +608,13 @@ __global__ void k_spread(const AtomArgs A) {
 }
 
 // Four lanes per atom, lane s taking the B-spline planes i3 = s, s+4, s+8
-// of the p^3 grid points; the partial sums meet by shuffles.
+// of the p^3 grid points; the partial sums meet by shuffles.  A derivative's
+// weights add up to 0, so its sums run over the potential's differences from
+// the row's, plane's or atom's first value: the potential itself, larger than
+// what is left of it, and the weights' rounding drop out.  Forces against 64
+// bits, mean of 8 sets of 9,000 charges on 48^3, order 4: 4.9e-7 relative,
+// 5.4e-7 without the differences (5.2e-7 with an x line of its own in each
+// transform); 60,000 on 90 x 80 x 96, order 6: 5.8e-7, 6.1e-7 and 6.1e-7.
 constexpr int GATHER_LANES = 4;
 
 template <int P>
@@ -623,6 +629,12 @@ __global__ void k_gather(const AtomArgs A) {
   if (t < A.natom) frac_coord(A, t, fr);
   const bool active = t < A.natom && frac_ok(A, fr);
   float f1 = 0.f, f2 = 0.f, f3 = 0.f, phi = 0.f;
+  constexpr int PP = P > 0 ? P : MAXORD;
+  constexpr int NC = (PP + GATHER_LANES - 1) / GATHER_LANES;
+  // the lane's planes: potential weighted along x and y, derivative weight
+  float pl[NC], pd[NC];
+#pragma unroll
+  for (int c = 0; c < NC; c++) pl[c] = pd[c] = 0.f;
   if (active) {
     float th1[MAXORD], th2[MAXORD], th3[MAXORD], d1[MAXORD], d2[MAXORD], d3[MAXORD];
     bspline<P>((float)(fr[0] - (int)fr[0]), p, th1, d1);
@@ -632,40 +644,57 @@ __global__ void k_gather(const AtomArgs A) {
     // spline values picked from the arrays by constant indices, so every
     // lane of the warp runs its own plane at once (a loop over all planes
     // that skipped the others' ran each plane with a quarter of the lanes)
-    constexpr int PP = P > 0 ? P : MAXORD;
 #pragma unroll
-    for (int c = 0; c < (PP + GATHER_LANES - 1) / GATHER_LANES; c++) {
+    for (int c = 0; c < NC; c++) {
       const int i3 = sub + c * GATHER_LANES;
       if (i3 >= p) break;
-      float t3 = 0.f, dd3 = 0.f;
+      float t3 = 0.f;
 #pragma unroll
       for (int q = 0; q < PP; q++)
         if (q == i3) {
           t3 = th3[q];
-          dd3 = d3[q];
+          pd[c] = d3[q];
         }
       const int kk = gidx((int)fr[2] - p + 1 + i3, A.n3);
+      float a1 = 0.f, a2 = 0.f, s20 = 0.f;
+      // a plane's values up to order 6 are all asked for before the first is used
+      constexpr int RW = P > 0 && P <= 6 ? P : 1;
+      float qv[RW][PP];
+      auto load_row = [&](int i2, float* q) {
+        const int jj = gidx((int)fr[1] - p + 1 + i2, A.n2);
+        const float* row = A.rg + ((size_t)kk * A.n2 + jj) * A.n1;
+#pragma unroll
+        for (int i1 = 0; i1 < PP; i1++) q[i1] = P > 0 || i1 < p ? row[gidx((int)fr[0] - p + 1 + i1, A.n1)] : 0.f;
+      };
+      if constexpr (RW > 1)
+#pragma unroll
+        for (int i2 = 0; i2 < RW; i2++) load_row(i2, qv[i2]);
 #pragma unroll
       for (int i2 = 0; i2 < (P > 0 ? P : MAXORD); i2++) {
         if (P == 0 && i2 >= p) break;
-        const int jj = gidx((int)fr[1] - p + 1 + i2, A.n2);
-        const float* row = A.rg + ((size_t)kk * A.n2 + jj) * A.n1;
-        float s1 = 0.f, s2 = 0.f, s3 = 0.f;
+        const int r = RW > 1 ? i2 : 0;
+        if constexpr (RW == 1) load_row(i2, qv[0]);
+        float s1 = 0.f, s2 = 0.f;
 #pragma unroll
-        for (int i1 = 0; i1 < (P > 0 ? P : MAXORD); i1++) {
+        for (int i1 = 0; i1 < PP; i1++) {
           if (P == 0 && i1 >= p) break;
-          const float qv = row[gidx((int)fr[0] - p + 1 + i1, A.n1)];
-          s1 += d1[i1] * qv;
-          s2 += th1[i1] * qv;
+          s1 += d1[i1] * (qv[r][i1] - qv[r][0]);
+          s2 += th1[i1] * qv[r][i1];
         }
-        s3 = s2;
-        phi += s2 * th2[i2] * t3;
-        f1 += s1 * th2[i2] * t3;
-        f2 += s2 * d2[i2] * t3;
-        f3 += s3 * th2[i2] * dd3;
+        if (i2 == 0) s20 = s2;
+        a1 += s1 * th2[i2];
+        a2 += (s2 - s20) * d2[i2];
+        pl[c] += s2 * th2[i2];
       }
+      phi += pl[c] * t3;
+      f1 += a1 * t3;
+      f2 += a2 * t3;
     }
   }
+  const float pl0 = __shfl_sync(0xffffffffu, pl[0], (threadIdx.x & 31) & ~(GATHER_LANES - 1));
+#pragma unroll
+  for (int c = 0; c < NC; c++)
+    if (sub + c * GATHER_LANES < p) f3 += (pl[c] - pl0) * pd[c];
 #pragma unroll
   for (int o = 1; o < GATHER_LANES; o <<= 1) {
     f1 += __shfl_xor_sync(0xffffffffu, f1, o);

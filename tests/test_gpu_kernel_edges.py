@@ -311,3 +311,27 @@ def test_a_coordinate_that_is_no_number(group_size, value, variant):
         assert all(v.sum() > s.ntap // 2 for v in far.values())
         assert masked or group_size == 8 or a == s.ntap - 1
     g.close()
+
+
+def test_reciprocal_forces_keep_their_precision():
+    """Two real x lines share one transform, which costs some of its rounding:
+    the forces are no further from 64 bits than with a line of its own in each
+    (5.21e-7, mean over 8 sets of charges of the same kind, standard error 1e-8),
+    the cheaper transform's loss of 3% made up for in the gather."""
+    from orac_b200 import units
+    from orac_b200.engine import Engine
+
+    s = systems.two_waters()
+    g, o = Engine(s.copy()), oracle.Oracle(s.copy())
+    err = []
+    for seed in range(8):
+        rng = np.random.default_rng([seed, 5])
+        n = 9000
+        edge = (n / 0.1) ** (1.0 / 3.0)
+        x = rng.uniform(-0.5, 0.5, (3, n)) * edge
+        q = rng.normal(0.0, 0.4, n)
+        q = (q - q.mean()) * units.charge_internal(1.0)
+        a = (x[0], x[1], x[2], q, np.eye(3) / edge, edge ** 3, 0.35, 4, (48, 48, 48))
+        err.append(rel_rms(g.do_pmesh_kspace(*a)[0], o.do_pmesh_kspace(*a)[0]))
+    assert np.mean(err) <= 5.21e-7, err
+    g.close()
