@@ -528,9 +528,12 @@ int orac_gpu_server_stats(orac_gpu_server* s, int64_t* out8);
  * reference) ---------------------------------------------------------------
  * Lanes per i group on the M shell and on the L/H shells (16 or 32; 16 only
  * for groups of at most 4 atoms) and resident blocks per SM of its
- * forces-only build (5, 6 or 8); 0 selects the default (5 blocks; half warps
- * on the M shell of contexts beside others and of large systems, whole warps
- * otherwise).  Forces, energies and trajectories do not depend on it: only
+ * forces-only build (5, 6 or 8; 3, 4 or 5 of the build that sums the work of
+ * a schedule, whose chains need the registers).  0 selects the default: whole
+ * warps (32) on the L/H shells, on the M shell of a context alone whose rows
+ * fit one wave of them, and along a schedule; half warps (16) on the other M
+ * shells; 6 blocks for a context alone whose rows fit one wave of 6 and not of
+ * 5, else 5.  Forces, energies and trajectories do not depend on it: only
  * speed does. */
 int orac_gpu_set_pair_tuning(orac_gpu_ctx* ctx, int lpg_m, int lpg_lh,
                              int minb);

@@ -112,12 +112,14 @@ int check_ready(orac_gpu_ctx* ctx) {
 // give the straight path the 96 registers it needs; 6 (80 registers) spills
 // and is slower with the device full (12 alchemical windows: 20.9 against
 // 19.9 ms for 12 steps), but takes the rows of 6 blocks per SM in one wave
-// (9,000 atoms, 750 blocks: 227 against 243 us a step).
-void pair_config(const orac_gpu_ctx* ctx, int* lpg, int* minb, bool m_shell) {
+// (9,000 atoms, 750 blocks: 227 against 243 us a step).  A launch that sums
+// the work of a schedule has its longest chains in the alchemical rows, which
+// whole warps shorten (14,900 atoms: 1.90 against 2.02 ms a 15-fs step).
+void pair_config(const orac_gpu_ctx* ctx, int* lpg, int* minb, bool m_shell, bool work) {
   const int blocks = (ctx->G + 3) / 4;
   const bool wave5 = blocks <= 5 * 148, wave6 = blocks <= 6 * 148;
   if (m_shell)
-    *lpg = ctx->tune_lpg_m ? ctx->tune_lpg_m : (!ctx->shared_device && wave6 ? 32 : 16);
+    *lpg = ctx->tune_lpg_m ? ctx->tune_lpg_m : (work || (!ctx->shared_device && wave6) ? 32 : 16);
   else
     *lpg = ctx->tune_lpg_lh ? ctx->tune_lpg_lh : 32;
   *minb = ctx->tune_minb ? ctx->tune_minb : (!ctx->shared_device && wave6 && !wave5 ? 6 : 5);
@@ -209,7 +211,6 @@ int shell_run_r(orac_gpu_ctx* ctx, char rshell, const ShellRadii& radii, const d
   a.natom = ctx->N;
   a.wcnt = ctx->d_wcnt;
   variant_fill(ctx, &a);
-  pair_config(ctx, &a.lpg, &a.minb, rshell == 'm');
   a.early = (flags & SH_RELEASE) ? orac_early(ctx) : 0;
   a.list_old = (flags & SH_LIST_OLD) ? 1 : 0;
   const bool want_e = (flags & SH_ENERGY) && d_e, want_s = (flags & SH_STRESS) && d_stress;
@@ -217,9 +218,7 @@ int shell_run_r(orac_gpu_ctx* ctx, char rshell, const ShellRadii& radii, const d
   a.stress = want_s ? 1 : 0;
   // the forces-only build sums force_alchemy's dwrk where a schedule asks
   a.dwrk = (a.variant == VAR_ALCH && !want_e && !want_s) ? ctx->pair_dwrk : nullptr;
-  // its longest chains are the alchemical rows, which whole warps shorten
-  // (14,900 atoms: 1.90 against 2.02 ms a 15-fs step)
-  if (a.dwrk && !ctx->tune_lpg_m) a.lpg = 32;
+  pair_config(ctx, &a.lpg, &a.minb, rshell == 'm', a.dwrk != nullptr);
   if (flags & SH_FIXED_OUT) a.ffix = reinterpret_cast<unsigned long long*>(d_f);
   if (want_e || want_s) CK(cudaMemsetAsync(ctx->d_acc, 0, ACC_N * sizeof(double), ctx->stream));
   if (!(flags & SH_PREPPED))

@@ -641,7 +641,7 @@ int bonded_launch(orac_gpu_ctx* ctx, int mask, const double* d_x, double* d_f, u
 void bonded_free(orac_gpu_ctx* ctx);
 int bonded_set_constraints(orac_gpu_ctx* ctx, const int* cnst, int ncnst);
 // api.cu
-void pair_config(const orac_gpu_ctx* ctx, int* lpg, int* minb, bool m_shell);
+void pair_config(const orac_gpu_ctx* ctx, int* lpg, int* minb, bool m_shell, bool work);
 int shell_run(orac_gpu_ctx* ctx, char rshell, const double* d_xyz,
               const double* d_grp, const double* d_mol, double* d_f,
               double* d_e, double* d_stress, int energy);

@@ -96,8 +96,9 @@ int orac_gpu_set_pair_tuning(orac_gpu_ctx* ctx, int lpg_m, int lpg_lh, int minb)
 int orac_gpu_get_pair_tuning(orac_gpu_ctx* ctx, int* out3) {
   if (!ctx || !out3) return ORAC_ERR_PARAM;
   int minb = 0;
-  pair_config(ctx, &out3[0], &minb, true);
-  pair_config(ctx, &out3[1], &minb, false);
+  const bool work = ctx->variant == VAR_ALCH && ctx->ne.on;
+  pair_config(ctx, &out3[0], &minb, true, work);
+  pair_config(ctx, &out3[1], &minb, false, work);
   out3[2] = minb;
   return ORAC_OK;
 }

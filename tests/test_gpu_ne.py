@@ -201,3 +201,33 @@ def test_schedule_on_another_grid():
     assert abs(g.md_work()[0] - f.md_work()[0]) <= 5e-3 * abs(f.md_work()[0])
     f.close()
     g.close()
+
+
+def test_pair_kernel_configuration_along_a_schedule():
+    """The configuration in effect: whole warps on the M shell by default, and
+    a caller's choice for the L/H shells or the M shell as it was made."""
+    def make():
+        s = systems.ligand_in_water(nlig=13, nwat=1000, box=31.3, nfft=(32, 32, 32))
+        s.ncell = (systems.linked_cells_for(31.3, s.shells),) * 3
+        g = Engine(s)
+        g.set_alchemy(s.ss_alchemy, 0.5, 0.5)
+        g.set_lambda(0.0, 0.0, 0.0, 0.0)
+        g.set_schedule(TIMES, LAMS["ladded"], LAMS["laddedq"], LAMS["lremoved"], LAMS["lremovedq"])
+        g.md_setup(SCHED["dt_h"], SCHED["lrespa"], SCHED["mrespa"], SCHED["nupdte"], SCHED["rshk"],
+                   n1respa=SCHED["n1respa"], n0respa=SCHED["n0respa"])
+        return g
+
+    engines = [make(), make()]
+    b = Batch(engines)  # (half warps are a batch's default without a schedule)
+    g = engines[0]
+    assert g.pair_tuning() == (32, 32, 5)
+    g.set_pair_tuning(0, 16, 0)
+    assert g.pair_tuning() == (32, 16, 5)
+    g.set_pair_tuning(16, 16, 6)
+    assert g.pair_tuning() == (16, 16, 6)
+    b.close()
+    for e in engines:
+        e.md_run(1)
+    assert np.array_equal(engines[0].md_state()[0], engines[1].md_state()[0])
+    for e in engines:
+        e.close()
