@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(128) k_pairs(const ListArgs A) {
   auto gather = [&](auto&& put) {
     int total = 0;
     if (A.allpairs) {
-      for (int l0 = 0; l0 < A.G; l0 += 32) {
+      for (int l0 = i + 1; l0 < A.G; l0 += 32) {
         const int l = l0 + lane;
         const bool hit = l < A.G && pair_in(A, xi, yi, zi, i, l);
         const unsigned bal = __ballot_sync(FULL, hit);
