@@ -526,8 +526,10 @@ static inline int dev_alloc(orac_gpu_ctx* ctx, T** p, size_t n) {
 // Kernel launches of the library go through orac_launch: programmatic
 // dependent launch, so a kernel's blocks are scheduled while its predecessor
 // in the stream still runs (in captured graphs too) and wait on the device
-// for the predecessor's completion and memory (pdl_enter, the first thing
-// every kernel of the library does).
+// for the predecessor's completion and memory (pdl_enter).  Before that wait a
+// kernel writes nothing and reads only what no kernel writes, or what a kernel
+// before its predecessor wrote: the predecessor waited for that one before it
+// released this one, early (pdl_release) or by its end.
 template <typename... KArgs, typename... Args>
 static inline cudaError_t orac_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
                                       cudaStream_t stream, Args&&... args) {

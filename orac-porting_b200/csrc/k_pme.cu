@@ -205,6 +205,7 @@ struct GridArgs {
   float2* save;
   const float2* cross;
   int early;  // pdl_release
+  int tw_written;  // a kernel of this call writes the twiddles (the static entry point)
   // the z pass sums the energy and virial into eout (0: potential only)
   int sums;
   // the plane passes: the y axis' twiddles and plan beside tw and P (the x
@@ -222,12 +223,16 @@ __global__ void __launch_bounds__(FFT_THREADS) k_fft(const GridArgs A) {
   const int B = A.B;
   float2* a = sm;
   float2* b = sm + B * n;
-  // the line's twiddles, staged after the two line buffers (no kernel writes
-  // them: before the wait)
+  // the line's twiddles, staged after the two line buffers: before the wait
+  // where they are a plan's, which no kernel writes
   float2* tws = sm + 2 * B * n;
-  for (int e = threadIdx.x; e < n; e += blockDim.x) tws[e] = A.tw[e];
+  auto stage = [&]() {
+    for (int e = threadIdx.x; e < n; e += blockDim.x) tws[e] = A.tw[e];
+  };
+  if (!A.tw_written) stage();
   pdl_enter();
   pdl_release(A.early);
+  if (A.tw_written) stage();
   // line geometry
   int nlines, i0 = 0, j0 = 0, k0 = 0, nl;
   if (MODE == XF || MODE == XI) {
@@ -1254,6 +1259,7 @@ extern "C" int orac_gpu_pme_kspace_static(void* stream, int numatoms, const doub
   const double pif = (double)3.14159265358979323846f;  // scalar_sum's single-precision pi
   const double rk = rkcut > 0.0 ? rkcut : 1e9;
   G.sums = 1;
+  G.tw_written = 1;
   G.fac = (float)(pif * pif / (ewald_coeff * ewald_coeff));
   G.pivol = (float)(pif * volume);
   G.rkcut2 = 0.25 * rk * rk / (pif * pif);
