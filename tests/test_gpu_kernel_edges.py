@@ -1,8 +1,10 @@
 """GPU kernels at the sizes where their tiles end, against the FP64 oracle:
 the pair kernel's rows (one group pair to several passes, groups of up to 3,
-4 and 8 atoms, half and whole warps a row), the plane FFT (odd axes, one x line left over, planes too
-large for shared memory) and the plan kept for calls that bring their own
-grid.  Tolerances as in the other parity tests: forces relative RMS <= 1e-5
+4 and 8 atoms, half and whole warps a row, coordinates that are no number),
+the list's rows (beyond the shared buffer, beyond the list's capacity), the
+plane FFT (odd axes, one x line left over, planes too large for shared memory)
+and the plan kept for calls that bring their own grid; and what a context
+keeps from one topology to the next.  Tolerances as in the other parity tests: forces relative RMS <= 1e-5
 (FP32 pair and spline arithmetic), energies 1e-6 of the terms' magnitudes.
 """
 import numpy as np
@@ -48,8 +50,8 @@ def test_rows_of_few_groups(nwat):
 @pytest.mark.parametrize("group_size", [1, 3, 4, 5, 8])
 @pytest.mark.parametrize("lanes", [(16, 16), (32, 32)])
 def test_group_sizes_and_lanes(group_size, lanes):
-    """Chains cut in groups of 1 to 8 atoms in water: each build of the pair
-    kernel, with exclusion masks."""
+    """Chains cut in groups of 1 to 8 atoms in water, with exclusion masks: the
+    pair kernel's builds with energies and stress (those without: below)."""
     from orac_b200.engine import Engine
 
     s = systems.solvated_chains(2100, 31, group_size=group_size)
@@ -334,4 +336,137 @@ def test_reciprocal_forces_keep_their_precision():
         a = (x[0], x[1], x[2], q, np.eye(3) / edge, edge ** 3, 0.35, 4, (48, 48, 48))
         err.append(rel_rms(g.do_pmesh_kspace(*a)[0], o.do_pmesh_kspace(*a)[0]))
     assert np.mean(err) <= 5.21e-7, err
+    g.close()
+
+
+FORMS = {"soft": {}, "shift": dict(shifted=True, qshift=4.0, ljshift=0.35)}
+
+
+def _chains(group_size, box="cubic"):
+    """Chains in water; skewed: a sheared box, and some atoms of fixed mass."""
+    s = systems.solvated_chains(2100, 31, group_size=group_size)
+    s.ss_alchemy = np.where(np.arange(s.ntap) < 14, -2, np.where(np.arange(s.ntap) < 20, 2, 1)).astype(np.int32)
+    s.rematom = (np.arange(s.ntap) % 5 == 0).astype(np.uint8)
+    if box == "skewed":
+        s.co = s.co.copy()
+        s.co[0, 1], s.co[0, 2], s.co[1, 2] = 0.12 * s.co[0, 0], -0.08 * s.co[0, 0], 0.1 * s.co[0, 0]
+        s.mass = s.mass.copy()
+        s.mass[8:30] = 1e25
+        s.ncell = None
+    return s
+
+
+def _variant(e, variant):
+    if variant == "rem":
+        e.set_rem(e.s.rematom, 0, 0.7)
+    elif variant in FORMS:
+        e.set_alchemy(e.s.ss_alchemy, 0.5, 0.5, **FORMS[variant])
+        e.set_lambda(ladd=0.3, lrm=0.6, laddq=0.4, lrmq=0.7)
+
+
+@pytest.mark.parametrize("box", ["cubic", "skewed"])
+@pytest.mark.parametrize("variant", ["std", "rem", "soft", "shift"])
+@pytest.mark.parametrize("group_size", [3, 4, 5, 8])
+def test_builds_agree_bit_for_bit(group_size, variant, box):
+    """Every build of the pair kernel for a group size and a variant -- with
+    energies and without, half and whole warps, each number of blocks per SM --
+    gives the same forces, and those of the oracle; in a skewed box, and with
+    fixed masses, whose pairs alchemy skips."""
+    from orac_b200.engine import Engine
+
+    s = _chains(group_size, box)
+    o = oracle.Oracle(s.copy())
+    _variant(o, variant)
+    o.update_lists()
+    first = {}
+    cfgs = ((16, 16, 5), (32, 32, 5), (16, 32, 6), (32, 16, 8)) if group_size <= 4 else ((32, 32, 5),)
+    for cfg in cfgs:
+        g = Engine(s.copy())
+        _variant(g, variant)
+        g.set_pair_tuning(*cfg)
+        g.update_lists()
+        for energies in (False, True):
+            for sh in "mlh":
+                F = _shell_dev(g, sh, energies)
+                first.setdefault(sh, F)
+                assert np.array_equal(F, first[sh]), (sh, cfg, energies)
+        g.close()
+    for sh in "mlh":
+        assert rel_rms(first[sh], o.shell(sh)[0]) <= 1e-5, sh
+
+
+@pytest.mark.parametrize("form", sorted(FORMS))
+def test_energy_steps_do_not_change_a_schedules_trajectory(form):
+    """The build that sums the work of a schedule (plain steps) and the one
+    with energies (energy steps) give the same forces bit for bit."""
+    from orac_b200.engine import Engine
+
+    s = systems.ligand_in_water(nlig=13, nwat=1000, box=31.3, nfft=(32, 32, 32))
+    s.ncell = (systems.linked_cells_for(31.3, s.shells),) * 3
+    out = []
+    for every in (0, 1, 3):
+        g = Engine(s.copy())
+        g.set_alchemy(s.ss_alchemy, 0.5, 0.5, **FORMS[form])
+        g.set_lambda(0.0, 0.0, 0.0, 0.0)
+        g.set_schedule([0.0, 40.0, 80.0], [1.0] * 3, [1.0] * 3, [0.0, 0.0, 1.0], [0.0, 1.0, 1.0])
+        g.md_setup(4.0, 2, 4, 3, "l")
+        g.md_run(14, energy_every=every)
+        out.append(np.concatenate(g.md_state()))
+        g.close()
+    assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
+
+
+@pytest.mark.parametrize("cells", [True, False])
+def test_rows_longer_than_the_buffer(cells):
+    """Rows of up to 700 partners, by linked cells and from all pairs: beyond
+    the 512 that a warp gathers in shared memory."""
+    from orac_b200.engine import Engine
+
+    s = systems.water_box(nwat=1728, box=35.76, lattice=12, nfft=(40, 40, 40))
+    s.shells = systems.Shells(rcutm=4.5, rtolm=0.3, rneim=0.4, rcutl=7.0, rtoll=0.3, rneil=0.5, rcuth=16.0, rtolh=0.3,
+                              rneih=0.8)
+    s.ncell = (systems.linked_cells_for(35.76, s.shells),) * 3 if cells else None
+    o, g = oracle.Oracle(s.copy()), Engine(s.copy())
+    o.update_lists()
+    g.update_lists()
+    # rows of the lower index: the first groups' hold all their neighbours
+    c = np.stack(s.group_centres())
+    d = c[:, :8, None] - c[:, None, :]
+    d = np.einsum("ij,jab->iab", s.co, d - 2.0 * np.round(0.5 * d))
+    assert ((d ** 2).sum(0) < 17.1 ** 2).sum(1).max() - 8 > 512
+    pairs, _ = g.list_pairs()
+    for sh in "hlm":
+        assert pairs[sh] == len(o.lists[sh]) - s.ngrp, sh
+    for sh in "mlh":
+        F, Fr = _shell_dev(g, sh), o.shell(sh)[0]
+        assert rel_rms(F, Fr) <= 1e-5, sh
+    g.close()
+
+
+def test_list_that_outgrows_its_capacity_in_a_run():
+    """A state much denser than the one the lists were sized for: the rows that
+    find no room are left out and the run reports it, also from a step graph."""
+    from orac_b200.engine import Engine
+    from orac_b200.lib import OracGpuError
+
+    s = systems.water_box(nwat=1728, box=72.0, lattice=12, nfft=(48, 48, 48))
+    s.shells = systems.Shells(rcutm=4.0, rtolm=0.3, rneim=0.4, rcutl=6.0, rtoll=0.3, rneil=0.4, rcuth=8.0, rtolh=0.3,
+                              rneih=0.6)
+    s.ncell = (systems.linked_cells_for(72.0, s.shells),) * 3
+    g = Engine(s)
+    g.md_setup(1.0, 2, 2, 2, "l")
+    g.md_run(2)
+    x, v = g.md_state()
+    com = np.stack([np.bincount(s.atomp - 1, weights=s.mass * x[k]) / np.bincount(s.atomp - 1, weights=s.mass)
+                    for k in range(3)])
+    y = x + (0.65 - 1.0) * com[:, s.atomp - 1]  # (molecules as a whole, towards the box's centre)
+    assert g.lib.orac_gpu_md_set_state(g.ctx, *[a.ctypes.data for a in (*np.ascontiguousarray(y),
+                                                                       *np.ascontiguousarray(v))]) == 0
+    with pytest.raises(OracGpuError, match="neighbour list capacity"):
+        g.md_run(3)  # (lists are updated every second step, from the step before's centres)
+    # set up again for the state at hand, the run goes on
+    s.xyz_restart = np.ascontiguousarray(y)
+    g.md_setup(1.0, 2, 2, 2, "l")
+    g.md_run(3)
+    assert np.isfinite(g.md_state()[0]).all()
     g.close()
