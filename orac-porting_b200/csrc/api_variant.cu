@@ -271,6 +271,7 @@ int orac_gpu_set_rem(orac_gpu_ctx* ctx, const int* rematom, int kind, double rem
   ParamGenBump bump(ctx);  // kernels capture these values: step graphs are re-captured
   if (!ctx || !ctx->have_topo) return ctx ? ctx_fail(ctx, ORAC_ERR_STATE, "topology not set") : ORAC_ERR_PARAM;
   CK(cudaSetDevice(ctx->device));
+  CK(cudaDeviceSynchronize());  // steps queued here or by a batch read the selection that is replaced
   if (!rematom) {
     bump.arm();
     if (ctx->variant == VAR_REM) ctx->variant = VAR_STD;
@@ -311,6 +312,7 @@ int orac_gpu_set_alchemy(orac_gpu_ctx* ctx, const int* ss_alchemy, const double*
   ParamGenBump bump(ctx);  // kernels capture these values: step graphs are re-captured
   if (!ctx || !ctx->have_topo) return ctx ? ctx_fail(ctx, ORAC_ERR_STATE, "topology not set") : ORAC_ERR_PARAM;
   CK(cudaSetDevice(ctx->device));
+  CK(cudaDeviceSynchronize());  // steps queued here or by a batch read the selection that is replaced
   if (!ss_alchemy) {
     bump.arm();
     if (ctx->variant == VAR_ALCH) ctx->variant = VAR_STD;

@@ -124,3 +124,48 @@ def test_hrem_with_thermostats_keeps_the_segment_energy_in_its_column():
     h.close()
     for e in engines:
         e.close()
+
+
+def test_selection_replaced_while_steps_are_queued():
+    """A REM or alchemy selection that is set or dropped while steps are queued
+    (orac_gpu_md_run_async, a batch that was not waited for): those steps keep
+    the one they were queued with."""
+    import ctypes as C
+
+    from orac_b200.engine import Batch
+
+    s = systems.ligand_in_water(nlig=13, nwat=1000, box=31.3, nfft=(32, 32, 32))
+    s.ncell = (systems.linked_cells_for(31.3, s.shells),) * 3
+    rem = (s.ss_alchemy == -2).astype(np.uint8)
+
+    def make():
+        g = Engine(s.copy())
+        g.set_rem(rem, 0, 0.5)
+        g.md_setup(4.0, 2, 4, 6, "l")
+        return g
+
+    ref = make()
+    ref.md_run(60)
+    x = ref.md_state()[0]
+    ref.close()
+    def drop(g):
+        f = C.cast(g.lib.orac_gpu_set_rem, C.CFUNCTYPE(C.c_int, C.c_void_p, C.c_void_p, C.c_int, C.c_double))
+        assert f(g.ctx, None, 0, 1.0) == 0
+
+    for replace in (drop, lambda g: g.set_rem(1 - rem, 1, 0.9),
+                    lambda g: g.set_alchemy(s.ss_alchemy, 0.5, 0.5)):
+        g = make()
+        assert g.lib.orac_gpu_md_run_async(g.ctx, 60) == 0
+        replace(g)
+        assert np.array_equal(g.md_state()[0], x)
+        g.close()
+    engines = [make(), make()]
+    b = Batch(engines)
+    b.run(60, sync=False)
+    drop(engines[0])
+    b.sync()
+    for e in engines:
+        assert np.array_equal(e.md_state()[0], x)
+    b.close()
+    for e in engines:
+        e.close()
