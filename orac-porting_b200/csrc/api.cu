@@ -111,10 +111,13 @@ int check_ready(orac_gpu_ctx* ctx) {
 // than a wave cost a launch half as much again.  5 blocks of 4 warps per SM
 // give the straight path the 96 registers it needs; 6 (80 registers) spills
 // and is slower with the device full (12 alchemical windows: 20.9 against
-// 19.9 ms for 12 steps), but takes the rows of 6 blocks per SM in one wave
-// (9,000 atoms, 750 blocks: 227 against 243 us a step).  A launch that sums
-// the work of a schedule has its longest chains in the alchemical rows, which
-// whole warps shorten (14,900 atoms: 1.90 against 2.02 ms a 15-fs step).
+// 19.9 ms for 12 steps), but takes the rows of 6 blocks per SM in one wave: a
+// step of 9,000 atoms (750 blocks) 293 against 301 us with the L2 flushed, of
+// 10,000 and 10,500 in chains (835, 877) 272 against 295 and 288 against 302;
+// water at the line's end is the exception (10,560 atoms, 880: 226 against
+// 206).  A launch that sums the work of a schedule has its longest chains in
+// the alchemical rows, which whole warps shorten (14,900 atoms: 1.90 against
+// 2.02 ms a 15-fs step).
 void pair_config(const orac_gpu_ctx* ctx, int* lpg, int* minb, bool m_shell, bool work) {
   const int blocks = (ctx->G + 3) / 4;
   const bool wave5 = blocks <= 5 * 148, wave6 = blocks <= 6 * 148;
