@@ -139,7 +139,10 @@ int orac_gpu_fft_pme(orac_gpu_ctx* ctx, const double* xp, const double* yp,
 /* do_pmesh_kspace: the SPME core on Cartesian coordinates with an explicit
  * recip (= 0.5 oc^T in ORAC), volume, alpha, order and grid.  dx/dy/dz are
  * accumulated, eer and virial set.  Uses the context's stream and buffers but
- * not its topology (charges are passed). */
+ * not its topology (charges are passed).  A grid or order other than the
+ * context's own is laid out on its first call and kept, in device memory that
+ * orac_gpu_footprint counts, until a call with another one or the context's
+ * end. */
 int orac_gpu_do_pmesh_kspace(orac_gpu_ctx* ctx, int numatoms, const double* x,
                              const double* y, const double* z,
                              const double* charge, const double* recip,
