@@ -145,7 +145,11 @@ int alch_upload_tables(orac_gpu_ctx* ctx) {
 }
 
 int variant_topology(orac_gpu_ctx* ctx, bool same_atoms) {
-  if (same_atoms) return ctx->h_vflag.empty() ? ORAC_OK : build_vflag(ctx);  // (fixed masses may differ)
+  if (same_atoms) {  // (fixed masses and charges may differ)
+    if (!ctx->h_vflag.empty())
+      if (int rc = build_vflag(ctx)) return rc;
+    return ctx->h_ssal.empty() ? ORAC_OK : upload_alch_charges(ctx, ctx->d_dq ? ctx->dlam : nullptr);
+  }
   ctx->variant = VAR_STD;
   ctx->h_rem.clear();
   ctx->h_ssal.clear();
@@ -383,6 +387,7 @@ int orac_gpu_set_lambda(orac_gpu_ctx* ctx, const double* lam, int intramol, int 
   alch_set(T.fq0, lam[6], lam[7], intramol, ljintra, 1);
   alch_set_d(T.df, lam[0], lam[1], d[0], d[1], intramol, ljintra, 0);
   alch_set_d(T.dfq, lam[2], lam[3], d[2], d[3], intramol, ljintra, 1);
+  for (int k = 0; k < 4; k++) ctx->dlam[k] = d[k];
   if (int rc = alch_upload_tables(ctx)) return rc;
   return upload_alch_charges(ctx, dlam);
 }

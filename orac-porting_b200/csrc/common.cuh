@@ -403,6 +403,7 @@ struct orac_gpu_ctx {
   BondedDev bd;
   std::vector<int> h_ssal;            // ss_alchemy
   double lam[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // ladd lrm laddq lrmq and the lambda0 set
+  double dlam[4] = {0, 0, 0, 0};  // the rates that came with them (where d_dq is set)
   double* d_qc = nullptr;  // [N] PME charges at lambda: (1 - |lambdaq_i|) q_i
   double* d_q0 = nullptr;  // [N] PME charges at lambda0
   double* d_dq = nullptr;  // [N] d(PME charge)/d(control lambda), or null

@@ -176,6 +176,8 @@ def _same_as_fresh(g, s, setup):
         # (energies and stress: FP64 sums of atomics, in any order)
         assert np.allclose(g.ue6(eg), f.ue6(ef), rtol=1e-12, atol=1e-9)
         assert np.linalg.norm(sg - sf) <= 1e-10 * np.linalg.norm(sf)
+    # (fixed-point charge grid, one thread's sums after it)
+    assert np.array_equal(g.fft_pme()[0], f.fft_pme()[0])
     if s.has_intra():
         assert rel_rms(g.intra_n1()[0], f.intra_n1()[0]) <= 1e-12
     f.close()
@@ -224,6 +226,12 @@ def test_topologies_one_after_another():
     _same_as_fresh(g, ligand, alch)
     take(g, ligand)  # the same number of atoms: the selection stays
     _same_as_fresh(g, ligand, alch)
+    other = ligand.copy()  # other charges and a fixed mass
+    other.charge = 0.9 * other.charge
+    other.mass[5] = 1e25
+    take(g, other)
+    _same_as_fresh(g, other, alch)
+    take(g, ligand)
     g.md_setup(4.0, 2, 4, 6, "l")
     g.md_run(1)
     take(g, small)
