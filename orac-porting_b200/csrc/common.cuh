@@ -220,6 +220,7 @@ enum {
 
 struct PmePlan {
   bool ready = false;  // every buffer and table below is that of the grid and order
+  bool saves = false;  // cgsave is one of them
   int n1 = 0, n2 = 0, n3 = 0, order = 0;
   int h1 = 0;
   float2* tw1 = nullptr;  // twiddles exp(-2 pi i k / n) per axis

@@ -833,7 +833,6 @@ int pme_setup(orac_gpu_ctx* ctx, int n1, int n2, int n3, int order) {
     return ctx_fail(ctx, ORAC_ERR_PARAM, "PME grid %dx%dx%d: sizes must factor into 2, 3, 5, 7", n1, n2, n3);
   if (P.ready && P.n1 == n1 && P.n2 == n2 && P.n3 == n3 && P.order == order) return ORAC_OK;
   P.ready = false;  // until every allocation below has succeeded
-  const bool saves = P.cgsave != nullptr;
   P.n1 = n1;
   P.n2 = n2;
   P.n3 = n3;
@@ -855,7 +854,7 @@ int pme_setup(orac_gpu_ctx* ctx, int n1, int n2, int n3, int order) {
   const size_t ng = (size_t)n1 * n2 * n3;
   const size_t nc = (size_t)P.h1 * n2 * n3;
   if (dev_alloc(ctx, &P.qfix, ng) || dev_alloc(ctx, &P.rgrid, ng) || dev_alloc(ctx, &P.cgrid, nc) ||
-      (saves && dev_alloc(ctx, &P.cgsave, nc)))
+      (P.saves && dev_alloc(ctx, &P.cgsave, nc)))
     return ORAC_ERR_CUDA;
   P.ready = true;
   return ORAC_OK;

@@ -254,8 +254,11 @@ int ne_init(orac_gpu_ctx* ctx, double tn0) {
   if (!ctx->d_ne && dev_alloc(ctx, &ctx->d_ne, 1)) return ORAC_ERR_CUDA;
   if (!ctx->d_ne_dq && dev_alloc(ctx, &ctx->d_ne_dq, N)) return ORAC_ERR_CUDA;
   {
-    const PmePlan& P = ctx->pme;
-    if (P.ready && !P.cgsave && dev_alloc(ctx, &ctx->pme.cgsave, (size_t)P.h1 * P.n2 * P.n3)) return ORAC_ERR_CUDA;
+    PmePlan& P = ctx->pme;
+    if (P.ready && !P.saves) {
+      if (dev_alloc(ctx, &P.cgsave, (size_t)P.h1 * P.n2 * P.n3)) return ORAC_ERR_CUDA;
+      P.saves = true;
+    }
   }
   if (dev_alloc(ctx, &ctx->d_ne_alist, al.size())) return ORAC_ERR_CUDA;
   ctx->ne_nal = (int)al.size();
