@@ -565,6 +565,7 @@ __device__ __forceinline__ void pdl_release(int early) {
 
 // ------------------------------------------------------ internal drivers
 // k_list.cu
+int list_reserve(orac_gpu_ctx* ctx, int64_t cap);
 int list_build_cells(orac_gpu_ctx* ctx, double rcut, GList* out);
 int list_build_allpairs(orac_gpu_ctx* ctx, double rcut, GList* out);
 int list_ensure_rows(orac_gpu_ctx* ctx, GList* L, const GList* parent);

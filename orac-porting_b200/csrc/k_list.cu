@@ -412,6 +412,23 @@ int pairs_launch(orac_gpu_ctx* ctx, const ListArgs& A) {
   return ORAC_OK;
 }
 
+}  // namespace
+
+// Room for `cap` entries in the H list and in the two that nest in its rows.
+// Their capacity is 0 until every allocation has succeeded.
+int list_reserve(orac_gpu_ctx* ctx, int64_t cap) {
+  for (GList& L : ctx->lists) {
+    L.cap = 0;
+    L.valid = false;
+  }
+  for (GList& L : ctx->lists)
+    if (dev_alloc(ctx, &L.j, cap) || dev_alloc(ctx, &L.mask, cap)) return ORAC_ERR_CUDA;
+  for (GList& L : ctx->lists) L.cap = cap;
+  return ORAC_OK;
+}
+
+namespace {
+
 // build, and once more where the list had to grow to the length found
 int pairs_build(orac_gpu_ctx* ctx, ListArgs A, GList* out) {
   for (;;) {
@@ -423,17 +440,7 @@ int pairs_build(orac_gpu_ctx* ctx, ListArgs A, GList* out) {
     out->npairs = total;
     if (total <= out->cap) break;
     const int64_t cap = total + total / 4 + 1024;
-    if (dev_alloc(ctx, &out->j, cap)) return ORAC_ERR_CUDA;
-    if (dev_alloc(ctx, &out->mask, cap)) return ORAC_ERR_CUDA;
-    out->cap = cap;
-    // nested lists share the rows of this list and need the same capacity
-    for (int q = 1; q < 3; q++) {
-      GList& L = ctx->lists[q];
-      if (dev_alloc(ctx, &L.j, cap)) return ORAC_ERR_CUDA;
-      if (dev_alloc(ctx, &L.mask, cap)) return ORAC_ERR_CUDA;
-      L.cap = cap;
-      L.valid = false;
-    }
+    if (int rc = list_reserve(ctx, cap)) return rc;
     A.cap = cap;
     A.j = out->j;
     A.mask = out->mask;

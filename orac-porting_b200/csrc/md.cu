@@ -2803,13 +2803,7 @@ int orac_gpu_md_setup(orac_gpu_ctx* ctx, const double* x, const double* y, const
     GList& H = ctx->lists[0];
     const int64_t want = H.npairs + H.npairs * 3 / 10 + 4096;
     if (H.cap < want) {
-      if (dev_alloc(ctx, &H.j, want) || dev_alloc(ctx, &H.mask, want)) return ORAC_ERR_CUDA;
-      H.cap = want;
-      for (int q = 1; q < 3; q++) {
-        GList& L = ctx->lists[q];
-        if (dev_alloc(ctx, &L.j, want) || dev_alloc(ctx, &L.mask, want)) return ORAC_ERR_CUDA;
-        L.cap = want;
-      }
+      if (int rc = list_reserve(ctx, want)) return rc;
       if (int rc = list_build_cells(ctx, rc_h, &ctx->lists[0])) return rc;
     }
   }
